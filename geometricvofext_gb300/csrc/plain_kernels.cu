@@ -3,7 +3,7 @@
 //
 //  K1 scanMixed          reconstruction::initialize      reconstruction.C:634-677
 //  K2 lsNormal           calcInterfaceNFromIsoAlphaGrad  reconstruction.C:85-141
-//  K3 planeSolve         cutCell::findSignedDistance     cutCell.C:611-799
+//  K3 planeSolve         (plane_solve.cu)
 //  K4 interfaceFlux      advection::timeIntegratedFlux   advection.C:85-221
 //  K5 update             upwind dVf + surfaceIntegrate + alpha update
 //                                                        advectionTemplates.C:371,399-406
@@ -95,45 +95,6 @@ __global__ void __launch_bounds__(128) kLsNormal(DevMesh m, const double* __rest
         st3(nrm, i, n / (mag(n) + kSMALL));
     }
     if (err) atomicOr(errOut, err);
-}
-
-// ---------------------------------------------------------------------------
-// K3: plane constant per mixed cell (cutCell::findSignedDistance), one
-// thread per cell.  On this FP64-poor part the kernel is limited by the
-// FP64 pipe, so the serial bracketing (the fewest cuts) with lanes kept
-// busy inside calcSubCell beats spreading the vertex levels over threads.
-// One instantiation per cell class (workspace caps K); a launch handles the
-// mixed cells of its class.
-// ---------------------------------------------------------------------------
-// With SPLIT the workspace is the splitWarpedFace one (warped faces as
-// triangle fans, the warped faces' centres among the vertex levels).
-template <class K, bool SPLIT>
-__global__ void __launch_bounds__(128) kPlaneSolve(DevMesh m, PlaneArgs p, int cls) {
-    const int nm = *p.nMixed;
-    uint32_t err = 0;
-    const int mask = SPLIT ? m.splitClassMask : m.classMask;
-    const uint8_t* cellCls = SPLIT ? m.splitClass : m.cellClass;
-    for (int i = spreadFirst(); i < nm; i += spreadStride()) {
-        const int c = p.mixed[i];
-        if (mask != (1 << cls) && cellCls[c] != cls) continue;
-        if (p.skip && p.skip[i]) continue;
-        CellWS<K> w;
-        double d = 0.0;
-        d3 ic = mk(0, 0, 0), is = mk(0, 0, 0);
-        int st;
-        if (!(SPLIT ? loadCellSplit(m, c, w) : loadCell(m, c, w))) {
-            err |= kErrSubFaceOverflow;
-            st = 1;
-        } else {
-            st = findSignedDistance(w, p.alpha[c], ld3(p.nrm, i), d, ic, is, err);
-        }
-        p.mStatus[i] = int8_t(st);
-        p.status[c] = int8_t(st);
-        p.dOut[i] = d;
-        st3(p.icOut, i, ic);
-        st3(p.isOut, i, is);
-    }
-    if (err) atomicOr(p.err, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -483,40 +444,6 @@ void launchScanMixed(const StepArgs& a, cudaStream_t st) {
 
 void launchLsNormal(const StepArgs& a, cudaStream_t st) {
     kLsNormal<<<residentGrid(kLsNormal, 128), 128, 0, st>>>(a.m, a.aCur, a.mixed, a.nMixed, a.nrm, a.err);
-}
-
-static PlaneArgs planeArgs(const StepArgs& a) {
-    PlaneArgs p;
-    p.alpha = a.aCur;
-    p.mixed = a.mixed;
-    p.nMixed = a.nMixed;
-    p.nrm = a.nrm;
-    p.mStatus = a.mStatus;
-    p.status = a.status;
-    p.dOut = a.dArr;
-    p.icOut = a.icArr;
-    p.isOut = a.isArr;
-    p.err = a.err;
-    p.skip = nullptr;
-    return p;
-}
-
-void launchPlaneSolve(const StepArgs& a, cudaStream_t st) { launchPlaneSolveSkip(a, nullptr, st); }
-
-void launchPlaneSolveSkip(const StepArgs& a, const uint8_t* skip, cudaStream_t st) {
-    PlaneArgs p = planeArgs(a);
-    p.skip = skip;
-    if (a.m.splitClassMask) {
-        const int mk = a.m.splitClassMask;
-        if (mk & 1) kPlaneSolve<CapsHex, true><<<residentGrid(kPlaneSolve<CapsHex, true>, 128), 128, 0, st>>>(a.m, p, 0);
-        if (mk & 2) kPlaneSolve<CapsPoly, true><<<residentGrid(kPlaneSolve<CapsPoly, true>, 128), 128, 0, st>>>(a.m, p, 1);
-        if (mk & 4) kPlaneSolve<CapsBig, true><<<residentGrid(kPlaneSolve<CapsBig, true>, 128), 128, 0, st>>>(a.m, p, 2);
-        return;
-    }
-    const int mk = a.m.classMask;
-    if (mk & 1) kPlaneSolve<CapsHex, false><<<residentGrid(kPlaneSolve<CapsHex, false>, 128), 128, 0, st>>>(a.m, p, 0);
-    if (mk & 2) kPlaneSolve<CapsPoly, false><<<residentGrid(kPlaneSolve<CapsPoly, false>, 128), 128, 0, st>>>(a.m, p, 1);
-    if (mk & 4) kPlaneSolve<CapsBig, false><<<residentGrid(kPlaneSolve<CapsBig, false>, 128), 128, 0, st>>>(a.m, p, 2);
 }
 
 void launchInterfaceUn0(const StepArgs& a, cudaStream_t st) {

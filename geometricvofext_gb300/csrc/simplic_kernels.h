@@ -169,6 +169,7 @@ void launchPlicPolygons(const StepArgs& a, int stride, double* pts, int* count, 
 void launchMapAlpha(const DevMesh& m, double* alpha, const double* normal, const double* distance, double lower,
                     double upper, uint32_t* err, cudaStream_t st);
 void launchLsNormal(const StepArgs& a, cudaStream_t st);
+PlaneArgs planeArgs(const StepArgs& a);
 void launchPlaneSolve(const StepArgs& a, cudaStream_t st);
 void launchInterfaceUn0(const StepArgs& a, cudaStream_t st);
 void launchInterfaceFaces(const StepArgs& a, cudaStream_t st);

@@ -263,6 +263,10 @@ struct Bracket {
     double lowD, upD, lowA, upA;
 };
 
+__device__ __forceinline__ bool absBelow(double x, double t) {  // fabs(x) < t, t > 0 (false for NaN)
+    return (bitsOf(x) & 0x7fffffffffffffffLL) < bitsOf(t);
+}
+
 // Newton on the cubic through the bracket (cutCell.C:743-789); returns the
 // plane constant.
 __device__ __forceinline__ double cubicDistance(const Bracket& br, double v13, double v23, double alphaI) {
@@ -274,13 +278,31 @@ __device__ __forceinline__ double cubicDistance(const Bracket& br, double v13, d
     const double c = 9.0 * a13 - 4.5 * a23 + 1.0 * alphaPrismatoid;
     const double dd = br.lowA - alphaI;
     double lambda = 0.5;
-    for (int iter = 0; iter < 100; ++iter) {
+    // Where the change never falls below TSMALL (one cell in a few hundred:
+    // the round-off of the cubic moves lambda further) the iterates go round a
+    // cycle, mostly of two, until the hundredth.  A cycle is found by keeping
+    // an iterate and comparing (Brent 1980), and only what is left of the
+    // hundred modulo its length is run: the same lambda.
+    double kept = lambda;
+    int keptAt = 0, limit = 100;
+    bool cycle = false;
+    for (int iter = 0; iter < limit; ++iter) {
         const double l2 = lambda * lambda;
         const double func = a * (lambda * l2) + b * l2 + c * lambda + dd;
         const double funcPrime = 3.0 * a * l2 + 2.0 * b * lambda + c;
         const double lambdaNew = lambda - (func / funcPrime);
-        if (fabs(lambdaNew - lambda) < kTSMALL) break;
+        if (absBelow(lambdaNew - lambda, kTSMALL)) break;
         lambda = lambdaNew;
+        if (!cycle) {
+            const int done = iter + 1;
+            if (bitsOf(lambda) == bitsOf(kept)) {
+                cycle = true;
+                limit = done + (100 - done) % (done - keptAt);
+            } else if ((done & (done - 1)) == 0) {
+                kept = lambda;
+                keptAt = done;
+            }
+        }
     }
     return br.lowD - lambda * (br.lowD - br.upD);
 }

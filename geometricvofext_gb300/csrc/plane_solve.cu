@@ -2,15 +2,16 @@
 // cutCell.C:611-799), a group of lanes per cell (plane_group.cuh).  Built
 // with -fmad=false.
 //
-// One GB300, kernel time with one thread per cell -> with a group per cell
-// (deformation field; interface cells in brackets):
-//   24^3 hex (331) 0.861 -> 0.167 ms     33^3 hex (617) 0.880 -> 0.224 ms
-//   128^3 hex (30,189) 1.451 -> 1.345 ms 256^3 hex (35,452) 1.636 -> 1.628 ms
-//   96^3 warped hex (7,146) 0.985 -> 0.406 ms
-//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 ms
-// A few hundred cells are the chain of one cell; tens of thousands fill the
-// FP64 pipe, where both forms issue about as many warp instructions a cell,
-// so there is no size at which one thread per cell is the better form.
+// One GB300, kernel time with one thread per cell -> a group per cell -> with
+// the work left out that plane_group.cuh lists (deformation field; interface
+// cells in brackets):
+//   24^3 hex (331) 0.861 -> 0.167 -> 0.101 ms
+//   33^3 hex (617) 0.880 -> 0.224 -> 0.138 ms
+//   128^3 hex (30,189) 1.451 -> 1.345 -> 0.660 ms
+//   256^3 hex (35,452) 1.636 -> 1.628 -> 0.764 ms
+//   96^3 warped hex (7,146) 0.985 -> 0.406 -> 0.348 ms
+//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 -> 1.56 ms
+// At the large sizes the FP64 pipe is about 80% busy.
 #include "plane_group.cuh"
 #include "simplic_kernels.h"
 
@@ -27,8 +28,11 @@ constexpr int kPlaneThreads = 64;
 // One instantiation per cell class (workspace caps K, G lanes per cell); a
 // launch handles the mixed cells of its class.  With SPLIT the workspace is
 // the splitWarpedFace one.
+// Six blocks per SM (168 registers, a few spilled) against four (200
+// registers): 0.80 against 0.82 ms at 128^3, 0.35 against 0.44 on the warped
+// 96^3 mesh; eight blocks spill more and gain nothing.
 template <class K, int G, bool SPLIT>
-__global__ void __launch_bounds__(kPlaneThreads) kPlaneSolve(DevMesh m, PlaneArgs p, int cls) {
+__global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, PlaneArgs p, int cls) {
     __shared__ GroupShared<K, G> shared[kPlaneThreads / 32];
     constexpr int kCells = 32 / G;
     const int nm = *p.nMixed;
@@ -62,7 +66,8 @@ __global__ void __launch_bounds__(kPlaneThreads) kPlaneSolve(DevMesh m, PlaneArg
         d3 ic = mk(0, 0, 0), is = mk(0, 0, 0);
         const double alphaI = act ? p.alpha[c] : 0.0;
         const d3 nI = act ? ld3(p.nrm, i) : mk(0, 0, 0);
-        int st = groupSignedDistance(w, act && ok, alphaI, nI, d, ic, is, err);
+        const unsigned box = (act && !SPLIT) ? m.boxCorner[c] : 0u;
+        int st = groupSignedDistance(w, act && ok, box, alphaI, nI, d, ic, is, err);
         if (act && !ok) {
             err |= kErrSubFaceOverflow;
             st = 1;

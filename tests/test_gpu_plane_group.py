@@ -36,3 +36,25 @@ def test_planes_bitexact_on_rough_fields(kind, n, split):
             np.testing.assert_array_equal(x, y, err_msg=f"{name}: {what}")
         for x, y, what in zip(g.interface(), o.interface(), "NDCS"):
             np.testing.assert_array_equal(x, y, err_msg=f"{name}: interface{what}")
+
+
+@pytest.mark.parametrize("scale,offset", [((1, 1, 1), (0, 0, 0)), ((1, 0.01, 30), (-5, 0.3, 2)),
+                                          ((1e-4, 1e-4, 1e-4), (0, 0, 0)), ((1e-7, 1, 1), (0, 0, 0)),
+                                          ((1, 1, 1), (3e7, 0, 0)), ((2e-3, 3e-3, 1e-3), (1e4, -1e4, 0))])
+def test_box_shortcuts_bitexact(scale, offset):
+    """Box cells of any proportions, size and place: the axis-aligned faces'
+    short forms and the single precision level test keep the oracle's bits,
+    also where they have to give way to the full operations."""
+    m = mg.hex_mesh(6, metrics=False)
+    m.points = m.points * np.asarray(scale, float) + np.asarray(offset, float)
+    mg.compute_metrics(m)
+    rng = np.random.default_rng(5)
+    g, o = capi.Simplic(m), O.Oracle(m)
+    x = (m.C - m.C.mean(0)) / np.asarray(scale, float)
+    for name, a in (("random", rng.random(m.n_cells)), ("steep", rng.random(m.n_cells) ** 12),
+                    ("plane", np.clip(0.5 - x @ [3.0, 2.0, 1.0], 0, 1)), ("slab", np.clip(0.5 - 4 * x[:, 1], 0, 1)),
+                    ("tilted slab", np.clip(0.5 - x @ [1e-4, 4.0, 1e-7], 0, 1))):
+        g.reconstruct(a)
+        o.reconstruct(a)
+        for p, q, what in zip(g.interface(), o.interface(), "NDCS"):
+            np.testing.assert_array_equal(p, q, err_msg=f"{name}: interface{what}")

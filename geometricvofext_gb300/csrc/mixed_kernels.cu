@@ -8,7 +8,7 @@
 //     plane constant of its cuboid (the cut volume inverted region by region,
 //     checked against alpha); any other cell takes the reference's own steps
 //     (cutCell.C:611-799: the bracket of two vertex levels, the cubic through
-//     the 1/3 and 2/3 cuts, Newton on the cubic);
+//     the 1/3 and 2/3 cuts, Newton on the cubic), the plain form's kernel;
 //   * Simpson fluxes: the clipped face areas of cutFace::timeIntegratedArea
 //     (cutFace.C:392-506) in FP32 on face-local coordinates (points shifted
 //     by the face centre, plane constant shifted with them), fan sums with
@@ -334,49 +334,44 @@ __device__ bool boxPlane(d3 n, d3 lo, d3 hi, double alpha, double V, double& d, 
     return true;
 }
 
-// One instantiation per cell class (workspace caps K); a launch handles the
-// mixed cells of its class.
-template <class K>
-__global__ void __launch_bounds__(128) kPlaneSolveMixed(DevMesh m, PlaneArgs p, int cls) {
+// The closed form of the box cells, one thread per mixed cell; the positions
+// of the others (other shapes, and boxes the closed form hands back) go to
+// `rest` for the general solve (plane_solve.cu).
+__global__ void __launch_bounds__(128) kBoxPlanes(DevMesh m, PlaneArgs p, int* __restrict__ rest,
+                                                  int* __restrict__ nRest) {
     const int nm = *p.nMixed;
-    uint32_t err = 0;
-    for (int i = spreadFirst(); i < nm; i += spreadStride()) {
-        const int c = p.mixed[i];
-        if (m.classMask != (1 << cls) && m.cellClass[c] != cls) continue;
-        CellWS<K> w;
-        double d = 0.0;
-        d3 ic = mk(0, 0, 0), is = mk(0, 0, 0);
-        int st;
-        const double alphaI = p.alpha[c];
-        const d3 nI = ld3(p.nrm, i);
-        const unsigned bx = m.boxCorner[c];
-        if (bx && alphaI > 0.0 && alphaI < 1.0) {
-            const int p0 = m.cpOff[c];
-            const d3 lo = ld3(m.pts, m.cPts[p0 + ((bx >> 3) & 7)]), hi = ld3(m.pts, m.cPts[p0 + (bx & 7)]);
-            if (boxPlane(nI, lo, hi, alphaI, m.V[c], d, ic, is)) {
-                p.mStatus[i] = 0;
-                p.status[c] = 0;
-                p.dOut[i] = d;
-                st3(p.icOut, i, ic);
-                st3(p.isOut, i, is);
-                continue;
+    const int lane = threadIdx.x & 31;
+    const int stride = spreadStride();
+    for (int i0 = spreadFirst() - lane; i0 < nm; i0 += stride) {  // the same trips on every lane
+        const int i = i0 + lane;
+        bool left = i < nm;
+        if (left) {
+            const int c = p.mixed[i];
+            const double alphaI = p.alpha[c];
+            const unsigned bx = m.boxCorner[c];
+            if (bx && alphaI > 0.0 && alphaI < 1.0) {
+                const int p0 = m.cpOff[c];
+                const d3 lo = ld3(m.pts, m.cPts[p0 + ((bx >> 3) & 7)]), hi = ld3(m.pts, m.cPts[p0 + (bx & 7)]);
+                double d = 0.0;
+                d3 ic = mk(0, 0, 0), is = mk(0, 0, 0);
+                if (boxPlane(ld3(p.nrm, i), lo, hi, alphaI, m.V[c], d, ic, is)) {
+                    p.mStatus[i] = 0;
+                    p.status[c] = 0;
+                    p.dOut[i] = d;
+                    st3(p.icOut, i, ic);
+                    st3(p.isOut, i, is);
+                    left = false;
+                }
             }
         }
-        if (!loadCell(m, c, w)) {
-            err |= kErrSubFaceOverflow;
-            st = 1;
-        } else if (mag(nI) < kTSMALL) {
-            st = int(sgn(0.5 - alphaI));
-        } else {
-            st = findSignedDistance(w, alphaI, nI, d, ic, is, err);
+        const unsigned who = __ballot_sync(0xffffffffu, left);
+        if (who) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(nRest, __popc(who));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (left) rest[base + __popc(who & ((1u << lane) - 1u))] = i;
         }
-        p.mStatus[i] = int8_t(st);
-        p.status[c] = int8_t(st);
-        p.dOut[i] = d;
-        st3(p.icOut, i, ic);
-        st3(p.isOut, i, is);
     }
-    if (err) atomicOr(p.err, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -709,33 +704,19 @@ __global__ void __launch_bounds__(128) kInterfaceUn0Mixed(DevMesh m, const int* 
 
 }  // namespace
 
-static void planeSolveMixedAll(const DevMesh& m, const PlaneArgs& p, cudaStream_t st) {
-    if (m.classMask & 1)
-        kPlaneSolveMixed<CapsHex><<<residentGridM(kPlaneSolveMixed<CapsHex>, 128), 128, 0, st>>>(m, p, 0);
-    if (m.classMask & 2)
-        kPlaneSolveMixed<CapsPoly><<<residentGridM(kPlaneSolveMixed<CapsPoly>, 128), 128, 0, st>>>(m, p, 1);
-    if (m.classMask & 4)
-        kPlaneSolveMixed<CapsBig><<<residentGridM(kPlaneSolveMixed<CapsBig>, 128), 128, 0, st>>>(m, p, 2);
-}
-
 void launchLsNormalMixed(const StepArgs& a, cudaStream_t st) {
     kLsNormalMixed<<<residentGridM(kLsNormalMixed, 128), 128, 0, st>>>(a.m, a.aCur, a.mixed, a.nMixed, a.nrm, a.err);
 }
 
-void launchPlaneSolveMixed(const StepArgs& a, cudaStream_t st) {
-    PlaneArgs p;
-    p.alpha = a.aCur;
-    p.mixed = a.mixed;
-    p.nMixed = a.nMixed;
-    p.nrm = a.nrm;
-    p.mStatus = a.mStatus;
-    p.status = a.status;
-    p.dOut = a.dArr;
-    p.icOut = a.icArr;
-    p.isOut = a.isArr;
-    p.err = a.err;
-    p.skip = nullptr;
-    planeSolveMixedAll(a.m, p, st);
+void launchPlaneSolveMixed(const StepArgs& a, bool boxes, cudaStream_t st) {
+    if (!boxes) {  // no box cell in the mesh
+        launchPlaneSolve(a, st);
+        return;
+    }
+    // the downwind-face list is free until the advect that follows
+    int* rest = reinterpret_cast<int*>(a.dwList);
+    kBoxPlanes<<<residentGridM(kBoxPlanes, 128), 128, 0, st>>>(a.m, planeArgs(a), rest, a.nMixed + 1);
+    launchPlaneSolveRest(a, rest, a.nMixed + 1, st);
 }
 
 void launchInterfaceUn0Mixed(const StepArgs& a, cudaStream_t st) {

@@ -4,7 +4,6 @@
 //   cutFace::calcSubFace / calcSubFaceCentreAndArea   cutFace.C:37-96, 136-259
 //   cutFace::timeIntegratedFaceFlux / Area            cutFace.C:262-506
 //   cutCell::calcSubCell and helpers                  cutCell.C:37-137, 343-542
-//   cutCell::findSignedDistance                       cutCell.C:611-799
 // with the same floating-point operation order as the reference, so that a
 // translation unit built with -fmad=false reproduces the CPU results bit for
 // bit.  Work that does not change any result is skipped (sub-cell centres
@@ -241,22 +240,6 @@ __device__ __forceinline__ bool loadCell(const DevMesh& m, int c, CellWS<K>& w) 
     return true;
 }
 
-// Vertex distances -n.x of the cell points and their stable descending
-// order (cutCell.C:644-670).
-template <class K>
-__device__ __forceinline__ void vertexOrder(const CellWS<K>& w, d3 nI, double* vd, int* order) {
-    const int np = w.np;
-    for (int i = 0; i < np; ++i) vd[i] = -dot(nI, w.P[i]);
-    for (int i = 0; i < np; ++i) {
-        int j = i;
-        while (j > 0 && vd[order[j - 1]] < vd[i]) {
-            order[j] = order[j - 1];
-            --j;
-        }
-        order[j] = i;
-    }
-}
-
 // The bracket the bisection over vertex levels ends with (cutCell.C:682-719):
 // plane constants and VOF of the two levels that enclose alpha.
 struct Bracket {
@@ -435,65 +418,6 @@ static __device__ __noinline__ void calcSubCell(const CellWS<K>& w, d3 n, double
         out.status = -1;
         out.vof = 1.0;
     }
-}
-
-// cutCell::findSignedDistance (cutCell.C:611-799), splitWarpedFace = false.
-// d/ic/is are written exactly where the reference writes interfaceD/C/S.
-template <class K>
-__device__ __forceinline__ int findSignedDistance(const CellWS<K>& w, double alphaI, d3 nI, double& dOut, d3& icOut,
-                                                  d3& isOut, uint32_t& err) {
-    if (mag(nI) < kTSMALL) return int(sgn(0.5 - alphaI));
-    const int np = w.np;
-    double vd[K::kPts];
-    int order[K::kPts];
-    vertexOrder(w, nI, vd, order);
-    Bracket br;
-    br.lowD = vd[order[0]];
-    br.upD = vd[order[np - 1]];
-    br.lowA = 0.0;
-    br.upA = 1.0;
-    int lowLabel = 0, upLabel = np - 1;
-    SubCell sc;
-    while ((upLabel - lowLabel) > 1) {
-        const int midLabel = (upLabel + lowLabel + 1) >> 1;
-        const double midDistance = vd[order[midLabel]];
-        calcSubCell(w, nI, midDistance, sc, err);
-        const double midAlpha = sc.vof;
-        if (fabs(midAlpha - alphaI) < kTSMALL) {
-            dOut = midDistance;
-            icOut = sc.ic;
-            isOut = sc.is;
-            return sc.status;
-        }
-        if (midAlpha > alphaI) {
-            upLabel = midLabel;
-            br.upD = midDistance;
-            br.upA = midAlpha;
-        } else {
-            lowLabel = midLabel;
-            br.lowD = midDistance;
-            br.lowA = midAlpha;
-        }
-    }
-    if (fabs(br.lowD - br.upD) < kTSMALL) {
-        const double midDistance = 0.5 * (br.lowD + br.upD);
-        calcSubCell(w, nI, midDistance, sc, err);
-        dOut = midDistance;
-        icOut = sc.ic;
-        isOut = sc.is;
-        return sc.status;
-    }
-    const double deltaDistance = (br.upD - br.lowD) / 3.0;
-    calcSubCell(w, nI, br.lowD + deltaDistance, sc, err);
-    const double v13 = sc.vof;
-    calcSubCell(w, nI, br.lowD + 2.0 * deltaDistance, sc, err);
-    const double v23 = sc.vof;
-    const double distance0 = cubicDistance(br, v13, v23, alphaI);
-    calcSubCell(w, nI, distance0, sc, err);
-    dOut = distance0;
-    icOut = sc.ic;
-    isOut = sc.is;
-    return sc.status;
 }
 
 // |area| of a face polygon clipped by the plane (calcSubFace then

@@ -48,8 +48,9 @@ __global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, Plane
     // warps are dealt out one per block before any block gets a second
     const int warps = gridDim.x * (kPlaneThreads / 32);
     for (int q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; q * kCells < nm; q += warps) {
-        const int i = q * kCells + w.g;
-        bool act = i < nm;
+        const int k = q * kCells + w.g;
+        bool act = k < nm;
+        const int i = act && p.rest ? p.rest[k] : k;
         const int c = act ? p.mixed[i] : 0;
         if (act && mask != (1 << cls) && cellCls[c] != cls) act = false;
         if (act && p.skip && p.skip[i]) act = false;
@@ -133,14 +134,11 @@ PlaneArgs planeArgs(const StepArgs& a) {
     p.isOut = a.isArr;
     p.err = a.err;
     p.skip = nullptr;
+    p.rest = nullptr;
     return p;
 }
 
-void launchPlaneSolve(const StepArgs& a, cudaStream_t st) { launchPlaneSolveSkip(a, nullptr, st); }
-
-void launchPlaneSolveSkip(const StepArgs& a, const uint8_t* skip, cudaStream_t st) {
-    PlaneArgs p = planeArgs(a);
-    p.skip = skip;
+static void launchAll(const StepArgs& a, const PlaneArgs& p, cudaStream_t st) {
     // lanes per cell: the faces of the class (6 of hexahedra: five cells a
     // warp; 12 of polyhedra on a half-warp; the whole warp beyond)
     if (a.m.splitClassMask) {
@@ -154,6 +152,21 @@ void launchPlaneSolveSkip(const StepArgs& a, const uint8_t* skip, cudaStream_t s
     if (mk & 1) launchClass<CapsHex, 6, false>(a.m, p, 0, st);
     if (mk & 2) launchClass<CapsPoly, 16, false>(a.m, p, 1, st);
     if (mk & 4) launchClass<CapsBig, 32, false>(a.m, p, 2, st);
+}
+
+void launchPlaneSolve(const StepArgs& a, cudaStream_t st) { launchAll(a, planeArgs(a), st); }
+
+void launchPlaneSolveSkip(const StepArgs& a, const uint8_t* skip, cudaStream_t st) {
+    PlaneArgs p = planeArgs(a);
+    p.skip = skip;
+    launchAll(a, p, st);
+}
+
+void launchPlaneSolveRest(const StepArgs& a, const int* rest, const int* nRest, cudaStream_t st) {
+    PlaneArgs p = planeArgs(a);
+    p.rest = rest;
+    p.nMixed = nRest;
+    launchAll(a, p, st);
 }
 
 }  // namespace simplic

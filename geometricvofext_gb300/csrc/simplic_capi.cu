@@ -655,7 +655,7 @@ int allocState(simplic_handle* h) {
     h->aOldBuf = M.alloc<double>(nc);
     h->status = M.alloc<int8_t>(nc);
     h->mixed = M.alloc<int>(nc);
-    h->nMixed = M.alloc<int>(1);
+    h->nMixed = M.alloc<int>(2);
     h->nrm = M.alloc<double>(size_t(3) * nc);
     h->mStatus = M.alloc<int8_t>(nc);
     h->dArr = M.alloc<double>(nc);
@@ -736,7 +736,7 @@ int allocState(simplic_handle* h) {
                     (void*)b.candPm, (void*)b.readyQ})
         if (!p) return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (solver state)");
     if (h->ctrl.record_cut_faces && !h->cutMask) return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (cut mask)");
-    CK(h, cudaMemsetAsync(h->nMixed, 0, sizeof(int), h->stream));
+    CK(h, cudaMemsetAsync(h->nMixed, 0, 2 * sizeof(int), h->stream));
     CK(h, cudaMemsetAsync(h->devErr, 0, sizeof(uint32_t), h->stream));
     CK(h, cudaMemsetAsync(h->alphaPhi, 0, sizeof(double) * nf, h->stream));
     CK(h, cudaMemsetAsync(b.corr, 0, sizeof(double) * nf, h->stream));
@@ -856,7 +856,7 @@ int runReconstruct(simplic_handle* h) {
     const size_t evIdx = h->eventsUsed;
     nextEvents(h, 0);
     CK(h, cudaEventRecord(h->events[evIdx].a, h->stream));
-    CK(h, cudaMemsetAsync(h->nMixed, 0, sizeof(int), h->stream));
+    CK(h, cudaMemsetAsync(h->nMixed, 0, 2 * sizeof(int), h->stream));
     timedLaunch(h, kKScan, [&] { launchScanMixed(a, h->stream); });
     if (h->ctrl.precision == SIMPLIC_PRECISION_LEARNED) {
         if (!h->haveNet) return fail(h, SIMPLIC_ERR_STATE, "learned precision: no network loaded (simplic_set_network)");
@@ -873,10 +873,10 @@ int runReconstruct(simplic_handle* h) {
             launchLearnedGate(a, R, h->netX, h->netA, h->netY, 16, h->netGateTol, h->nLearned, h->stream);
         });
         CK(h, ne);
-        timedLaunch(h, kKPlane, [&] { launchPlaneSolveMixed(a, h->stream); });
+        timedLaunch(h, kKPlane, [&] { launchPlaneSolveMixed(a, h->nBoxCells > 0, h->stream); });
     } else if (h->ctrl.precision == SIMPLIC_PRECISION_MIXED) {
         timedLaunch(h, kKLs, [&] { launchLsNormalMixed(a, h->stream); });
-        timedLaunch(h, kKPlane, [&] { launchPlaneSolveMixed(a, h->stream); });
+        timedLaunch(h, kKPlane, [&] { launchPlaneSolveMixed(a, h->nBoxCells > 0, h->stream); });
     } else if (h->ctrl.orientation_method == SIMPLIC_ORIENTATION_ISO_RDF) {
         if (int r = runIsoRDF(h, a)) return r;
     } else {

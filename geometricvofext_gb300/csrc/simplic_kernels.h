@@ -33,7 +33,7 @@ struct StepArgs {
     // reconstruction state (compact, indexed by position in the mixed list)
     int8_t* status;   // [nc]
     int* mixed;       // [nc]
-    int* nMixed;      // [1]
+    int* nMixed;      // [0] mixed cells, [1] those the mixed forms' box planes left to the general solve
     double* nrm;      // [3 nc]
     int8_t* mStatus;  // [nc]
     double* dArr;     // [nc]
@@ -135,6 +135,7 @@ struct PlaneArgs {
     double* isOut;
     uint32_t* err;
     const uint8_t* skip;  // optional per mixed cell: nonzero keeps the previous plane (isoRDF)
+    const int* rest;      // optional list of mixed positions to solve, *nMixed of them
 };
 
 // Buffers of the isoRDF orientation (reconstruction.C:193-405), allocated
@@ -160,6 +161,8 @@ void launchScanMixed(const StepArgs& a, cudaStream_t st);
 void launchRdfStart(const StepArgs& a, const RdfBuffers& r, cudaStream_t st);
 void launchRdfNormals(const StepArgs& a, const RdfBuffers& r, cudaStream_t st);
 void launchPlaneSolveSkip(const StepArgs& a, const uint8_t* skip, cudaStream_t st);
+// the plane solve of the mixed positions rest[0 .. *nRest) only
+void launchPlaneSolveRest(const StepArgs& a, const int* rest, const int* nRest, cudaStream_t st);
 void launchRdfConstruct(const StepArgs& a, const RdfBuffers& r, cudaStream_t st);
 void launchRdfResidual(const StepArgs& a, const RdfBuffers& r, cudaStream_t st);
 // PLIC polygon of every mixed cell: up to `stride` points at pts[3 stride i],
@@ -183,7 +186,8 @@ void launchRecipVolume(const DevMesh& m, double* rV, cudaStream_t st);
 void launchStencilRows(const DevMesh& m, bool count, int* len, const int* off, int* rows, cudaStream_t st);
 // mixed-precision form (FP32 normals and Simpson clipping, FP64 volume matching)
 void launchLsNormalMixed(const StepArgs& a, cudaStream_t st);
-void launchPlaneSolveMixed(const StepArgs& a, cudaStream_t st);
+// boxes: the mesh has axis-aligned box cells
+void launchPlaneSolveMixed(const StepArgs& a, bool boxes, cudaStream_t st);
 void launchInterfaceUn0Mixed(const StepArgs& a, cudaStream_t st);
 void launchInterfaceFacesMixed(const StepArgs& a, cudaStream_t st);
 // learned-normal form (the mixed form with the network's normals)

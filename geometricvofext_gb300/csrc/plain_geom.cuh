@@ -11,6 +11,7 @@
 // the face alone and are computed once per cell).
 #pragma once
 
+#include "int_math.cuh"
 #include "simplic_device.cuh"
 
 namespace simplic {
@@ -600,10 +601,11 @@ __device__ __forceinline__ bool nonNegBits(long long b) {
 // w = 1 gives 1 x = x exactly; w = 0 gives 0 x + aN = aN exactly when aN is
 // a nonzero finite number and x is finite, and +0 when aN is +0.  For w = 1,
 // (aP - aN) + aN is aP itself when aN is +0 (aP not -0), when aP is +0 (the
-// sum cancels to +0), or when aP and aN share sign and binade (Sterbenz: the
-// difference is exact).  Other cases (a zero or non-finite value where the
-// sign of a zero decides, or aP, aN of different binades) take the
-// reference's arithmetic.  The tests are integer operations on the bits.
+// sum cancels to +0), when aP and aN share sign and binade (Sterbenz: the
+// difference is exact), or where upwindSettled shows it on the bits.  Other
+// cases (a zero or non-finite value where the sign of a zero decides, an aN
+// above aP or of the other sign) take the reference's arithmetic.  The tests
+// are integer operations on the bits.
 __device__ __forceinline__ double upwindAlpha(double ph, double aP, double aN) {
     const long long bp = bitsOf(ph), bP = bitsOf(aP), bN = bitsOf(aN);
     const long long kExp = 0x7ff0000000000000LL, kSign = (long long)0x8000000000000000ULL;
@@ -612,6 +614,8 @@ __device__ __forceinline__ double upwindAlpha(double ph, double aP, double aN) {
         if (finite && ((bN == 0 && bP != kSign) || bP == 0 ||
                        (((bP ^ bN) & (kSign | kExp)) == 0 && (bP & kExp) != 0)))
             return aP;
+        const int settled = upwindSettled(uint64_t(bP), uint64_t(bN));
+        if (settled) return settled > 0 ? aP : 0.0;
         return (aP - aN) + aN;
     }
     if (finite && (bN << 1) != 0) return aN;
@@ -636,16 +640,34 @@ __device__ __forceinline__ double fluxDt(double ph, double af, double dt, double
     return x * dt;
 }
 
+// (phi * alpha_f) * dt and, in q, that over dt (alphaPhi of the face): both
+// products and the quotient on the integer pipe where every value is a normal
+// number, else by fluxDt and a division through y = RN(1/dt).
+__device__ __forceinline__ double fluxDtQuot(double ph, double af, double dt, double y, double& q) {
+    uint64_t x = uint64_t(bitsOf(ph)), dv, qb;
+    const uint64_t ba = uint64_t(bitsOf(af)), bt = uint64_t(bitsOf(dt));
+    bool ok = true;
+    if (ba != 0x3ff0000000000000ull) ok = mulOnInts(x, ba, x);
+    if (ok && mulQuotOnInts(x, bt, dv, qb)) {
+        q = __longlong_as_double((long long)qb);
+        return __longlong_as_double((long long)dv);
+    }
+    double p;
+    bool prod;
+    const double v = fluxDt(ph, af, dt, p, prod);
+    q = prod ? divOfProduct(v, dt, y, p) : divByRecip(v, dt, y);
+    return v;
+}
+
 // dVf of one face before bounding: the Simpson value when the upwind cell is
 // cut, else (phi * alpha_f) * dt with alpha_f = w (aP - aN) + aN, w = pos0(phi)
 // (upwind weights through the linear interpolation formula); boundary faces
-// use the boundary value of alpha.  x / prod as for fluxDt (prod false for a
-// Simpson value).
+// use the boundary value of alpha.
 __device__ __forceinline__ double baseDVf(const DevMesh& m, int f, double ph, const double* aCur,
-                                          const int8_t* status, const double* dvfI, const double* alphaB, double dt,
-                                          double& x, bool& prod) {
+                                          const int8_t* status, const double* dvfI, const double* alphaB, double dt) {
     const bool pos = nonNegBits(bitsOf(ph));
-    prod = false;
+    double x;
+    bool prod;
     if (f < m.nfi) {
         const int o = m.own[f], nb = m.nei[f];
         const int up = pos ? o : nb;
@@ -656,12 +678,6 @@ __device__ __forceinline__ double baseDVf(const DevMesh& m, int f, double ph, co
     if (pos && status[o] == 0) return dvfI[f];
     const double ab = alphaB ? alphaB[f - m.nfi] : aCur[o];
     return fluxDt(ph, ab, dt, x, prod);
-}
-__device__ __forceinline__ double baseDVf(const DevMesh& m, int f, double ph, const double* aCur,
-                                          const int8_t* status, const double* dvfI, const double* alphaB, double dt) {
-    double x;
-    bool prod;
-    return baseDVf(m, f, ph, aCur, status, dvfI, alphaB, dt, x, prod);
 }
 
 }  // namespace simplic

@@ -220,17 +220,106 @@ __global__ void __launch_bounds__(128) kInterfaceFaces(DevMesh m, const int2* __
 // ---------------------------------------------------------------------------
 // K5: upwind flux, interface overrides, surfaceIntegrate and alpha update
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) kUpdate(DevMesh m, const double* __restrict__ phi,
-                                               const double* __restrict__ aCur, const double* __restrict__ aOld,
-                                               double* __restrict__ aNew, const int8_t* __restrict__ status,
-                                               const double* __restrict__ dvfI, const double* __restrict__ alphaB,
-                                               const double* __restrict__ Sp, const double* __restrict__ Su,
-                                               double dt, double rDeltaT, double rrDeltaT,
-                                               double* __restrict__ alphaPhi,
-                                               int* __restrict__ ovList, int* __restrict__ ovCount, int ovCap) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+struct UpdateArgs {
+    const double* phi;
+    const double* aCur;
+    const double* aOld;
+    double* aNew;
+    const int8_t* status;
+    const double* dvfI;
+    const double* alphaB;
+    const double* Sp;
+    const double* Su;
+    double dt, rDeltaT, rrDeltaT;
+    double* alphaPhi;
+    int* ovList;
+    int* ovCount;
+    int ovCap;
+};
+
+// dVf of face f of cell c (own: c owns it; nb: the cell across, -1 on the
+// boundary; ac, stC: c's alpha and status) and, for an owned face, dVf / dt
+// in q: the Simpson value when the upwind cell is cut, else the upwind flux.
+__device__ __forceinline__ double faceDVf(const DevMesh& m, const UpdateArgs& u, int f, bool own, int nb, double ac,
+                                          int8_t stC, double& q) {
+    const double ph = u.phi[f];
+    const bool pos = nonNegBits(bitsOf(ph));
+    double af;
+    bool cut;
+    if (nb >= 0) {
+        const double ax = u.aCur[nb];
+        cut = (pos == own ? stC : u.status[nb]) == 0;
+        af = cut ? 0.0 : upwindAlpha(ph, own ? ac : ax, own ? ax : ac);
+    } else {
+        cut = pos && stC == 0;
+        af = u.alphaB ? u.alphaB[f - m.nfi] : ac;
+    }
+    if (cut) {
+        const double dv = u.dvfI[f];
+        q = own ? divByRecip(dv, u.dt, u.rDeltaT) : 0.0;
+        return dv;
+    }
+    return fluxDtQuot(ph, af, u.dt, u.rDeltaT, q);
+}
+
+// The update of one cell.  What bounds it: in the first steps of a run, when
+// most cells and their neighbours hold exact zeros, the loads' latency and
+// HBM (64 B of traffic per cell); later, when almost every cell holds a small
+// remainder, the arithmetic of six upwind fluxes per cell, for which the
+// FP64 pipe (16 cycles per warp instruction) is the narrow one.  So:
+//   * an empty neighbourhood issues no FP64 at all (below);
+//   * the products of the fluxes and alphaPhi are formed on the integer pipe
+//     (fluxDtQuot), the FP64 pipe is left the sums, the upwind differences
+//     that are not settled on the bits, and the divisions by V and 1/dt;
+//   * TILE: on a lattice mesh a block is a tile of TX x TY x TZ cells and
+//     each flux inside the tile is formed once, by its owner, and read by the
+//     cell across from shared memory; the fluxes through the tile's low sides
+//     are one more flux for two thirds of the threads (3.6 fluxes per cell
+//     instead of 6).
+// Other meshes take one thread per cell in cell order (TX = TY = TZ = 0).
+// One GB300, before -> with the products on integers -> with tiles: 128^3 in
+// the middle of the deformation run 0.222 -> 0.174 -> 0.156 ms, 256^3 with
+// alpha spread over the mesh 2.05 -> 1.76 -> 1.07 ms (0.28 -> 0.29 -> 0.25 ms
+// in its first steps); 45^3 x 6 tetrahedra (no lattice) 0.048 -> 0.039 ms.
+// The FP64 pipe is 63% busy then, the issue slots 55%.  Other tiles, same
+// two cases: 8 x 8 x 4 0.168 and 1.14, 16 x 4 x 4 0.174 and 1.24, 32 x 4 x 2
+// 0.192 and 1.50 (more sides, or more warps at a barrier); 8 or 12 blocks of
+// 128 per SM instead of 10 lose 0.04 ms in the first steps.
+template <int TX, int TY, int TZ>
+struct UpdateBlock {
+    static constexpr int kThreads = TX ? TX * TY * TZ : 256;
+};
+template <int TX, int TY, int TZ>
+__global__ void __launch_bounds__((UpdateBlock<TX, TY, TZ>::kThreads), (1280 / UpdateBlock<TX, TY, TZ>::kThreads))
+    kUpdate(DevMesh m, UpdateArgs u) {
+    constexpr bool kTile = TX > 0;
+    constexpr int kThreads = UpdateBlock<TX, TY, TZ>::kThreads;
+    constexpr int kHz = TX * TY, kHy = TX * TZ, kHx = TY * TZ;  // faces on the tile's low sides
+    constexpr int kDx = kTile ? TX : 1, kDy = kTile ? TY : 1;    // (divisors)
+    __shared__ double sDv[kTile ? 3 : 1][kTile ? kThreads : 1];  // dVf of each cell's +x, +y, +z face
+    __shared__ double sLow[kTile ? kHz + kHy + kHx : 1];         // dVf through the low sides: z, y, x
+    __shared__ uint8_t sWork[kTile ? kThreads : 1];              // an interior cell on the arithmetic path
+    const int tid = threadIdx.x;
+    int c, li = 0, lj = 0, lk = 0, i = 0, j = 0, k = 0;
+    bool valid;
+    if (kTile) {
+        li = tid % kDx;
+        lj = tid / kDx % kDy;
+        lk = tid / (kDx * kDy);
+        i = blockIdx.x * TX + li;
+        j = blockIdx.y * TY + lj;
+        k = blockIdx.z * TZ + lk;
+        valid = i < m.latNx && j < m.latNy && k < m.latNz;
+        c = i + m.latNx * (j + m.latNy * k);
+    } else {
+        c = blockIdx.x * blockDim.x + tid;
+        valid = c < m.nc;
+    }
     bool ov = false, inSet = false;
-    if (c < m.nc) {
+    bool work = false, interior = false;
+    int k0 = 0, k1 = 0;  // slots in memory; an interior lattice cell: k0 its latticeBase
+    double ao = 0.0, ac = 0.0;
+    if (valid) {
         // The face-slot records: from the lattice formula for the interior
         // cells of a lattice mesh (no addressing read), else the first
         // kBatch from memory, loaded together so they are in flight at once;
@@ -238,15 +327,14 @@ __global__ void __launch_bounds__(256) kUpdate(DevMesh m, const double* __restri
         // slots hold x = -2.
         constexpr int kBatch = 6;
         int2 sl[kBatch];
-        int k0, k1;
-        if (m.latNx && latticeSlotsFast(c, m.latNx, m.latNy, m.latNz, m.latDivLayer, m.latDivNx, sl)) {
-            k0 = 0;
-            k1 = kBatch;
+        interior = kTile && latticeSlotsAt(c, i, j, k, i + m.latNx * j, m.latNx, m.latNy, m.latNz, sl);
+        if (interior) {
+            k0 = sl[3].y;
         } else {
             k0 = m.uniformFaces ? c * m.uniformFaces : m.cOff[c];
             k1 = m.uniformFaces ? k0 + m.uniformFaces : m.cOff[c + 1];
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j) sl[j] = (k0 + j < k1) ? m.cSlot[k0 + j] : make_int2(-2, 0);
+            for (int q = 0; q < kBatch; ++q) sl[q] = (k0 + q < k1) ? m.cSlot[k0 + q] : make_int2(-2, 0);
         }
         // Every load the common case needs is issued before any is used, so
         // a cell costs one memory round trip: the alpha across each slot
@@ -255,19 +343,19 @@ __global__ void __launch_bounds__(256) kUpdate(DevMesh m, const double* __restri
         double ax[kBatch];
         double pv[kBatch];
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-            ax[j] = 0.0;
-            if (sl[j].x >= 0)
-                ax[j] = aCur[sl[j].x];
-            else if (sl[j].x == -1 && alphaB)
-                ax[j] = alphaB[(sl[j].y & 0x7fffffff) - m.nfi];
-            pv[j] = (sl[j].x != -2 && sl[j].y >= 0) ? phi[sl[j].y] : 0.0;
+        for (int q = 0; q < kBatch; ++q) {
+            ax[q] = 0.0;
+            if (sl[q].x >= 0)
+                ax[q] = u.aCur[sl[q].x];
+            else if (sl[q].x == -1 && u.alphaB)
+                ax[q] = u.alphaB[(sl[q].y & 0x7fffffff) - m.nfi];
+            pv[q] = (sl[q].x != -2 && sl[q].y >= 0) ? u.phi[sl[q].y] : 0.0;
         }
-        const double ao = aOld[c];
-        const double ac = aCur[c];
+        ao = u.aOld[c];
+        ac = u.aCur[c];
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j)
-            if (sl[j].x == -1 && !alphaB) ax[j] = ac;  // zero-gradient boundary value
+        for (int q = 0; q < kBatch; ++q)
+            if (sl[q].x == -1 && !u.alphaB) ax[q] = ac;  // zero-gradient boundary value
         // Empty neighbourhood: every dVf is a signed zero, surfaceIntegrate
         // gives +0 and ((ao*r) - 0*r)/r returns ao itself (bit for bit), and
         // alphaPhi = dVf/dt is a zero with the sign of phi.  The zero tests
@@ -275,94 +363,146 @@ __global__ void __launch_bounds__(256) kUpdate(DevMesh m, const double* __restri
         // cells issue no FP64 instruction.
         const auto isZero = [](double x) { return (bitsOf(x) << 1) == 0; };
         const long long kSign = (long long)0x8000000000000000ULL;
-        bool quick = (Sp == nullptr) && (Su == nullptr) && isZero(ao) && isZero(ac);
+        bool quick = (u.Sp == nullptr) && (u.Su == nullptr) && isZero(ao) && isZero(ac);
         if (quick) {
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j) quick = quick && isZero(ax[j]);
-            for (int k = k0 + kBatch; quick && k < k1; ++k) {
-                const int2 s = m.cSlot[k];
-                const double x = (s.x >= 0) ? aCur[s.x] : (alphaB ? alphaB[(s.y & 0x7fffffff) - m.nfi] : ac);
+            for (int q = 0; q < kBatch; ++q) quick = quick && isZero(ax[q]);
+            for (int q = k0 + kBatch; quick && q < k1; ++q) {
+                const int2 s = m.cSlot[q];
+                const double x = (s.x >= 0) ? u.aCur[s.x] : (u.alphaB ? u.alphaB[(s.y & 0x7fffffff) - m.nfi] : ac);
                 quick = isZero(x);
             }
         }
         if (quick) {
-            aNew[c] = ao;
+            u.aNew[c] = ao;
             // owned faces only (the owner writes each face); an internal face's
             // alpha_f is +0, a boundary face's zero also carries alpha_b's sign
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j) {
-                if (sl[j].x == -2 || sl[j].y < 0) continue;
-                long long sgnBits = bitsOf(pv[j]) & kSign;
-                if (sl[j].x == -1) sgnBits ^= bitsOf(ax[j]) & kSign;
-                alphaPhi[sl[j].y] = __longlong_as_double(sgnBits);
+            for (int q = 0; q < kBatch; ++q) {
+                if (sl[q].x == -2 || sl[q].y < 0) continue;
+                long long sgnBits = bitsOf(pv[q]) & kSign;
+                if (sl[q].x == -1) sgnBits ^= bitsOf(ax[q]) & kSign;
+                u.alphaPhi[sl[q].y] = __longlong_as_double(sgnBits);
             }
-            for (int k = k0 + kBatch; k < k1; ++k) {
-                const int2 s = m.cSlot[k];
+            for (int q = k0 + kBatch; q < k1; ++q) {
+                const int2 s = m.cSlot[q];
                 if (s.y < 0) continue;
-                long long sgnBits = bitsOf(phi[s.y]) & kSign;
-                if (s.x < 0) sgnBits ^= bitsOf(alphaB ? alphaB[s.y - m.nfi] : ac) & kSign;
-                alphaPhi[s.y] = __longlong_as_double(sgnBits);
+                long long sgnBits = bitsOf(u.phi[s.y]) & kSign;
+                if (s.x < 0) sgnBits ^= bitsOf(u.alphaB ? u.alphaB[s.y - m.nfi] : ac) & kSign;
+                u.alphaPhi[s.y] = __longlong_as_double(sgnBits);
             }
-        } else {
-            // surfaceIntegrate in ascending face order: the batch, then the rest
-            double sum = 0.0;
-            const auto add = [&](int fa) {
-                const int f = fa & 0x7fffffff;
-                const double ph = phi[f];
-                double x;
-                bool prod;
-                const double dv = baseDVf(m, f, ph, aCur, status, dvfI, alphaB, dt, x, prod);
-                if (fa >= 0) {
-                    // dv / dt: from the product dv was made of when there is one
-                    alphaPhi[f] = prod ? divOfProduct(dv, dt, rDeltaT, x) : divByRecip(dv, dt, rDeltaT);
-                    sum += dv;
-                } else {
-                    sum -= dv;
-                }
-            };
+        }
+        work = !quick;
+    }
+    double sum = 0.0;  // surfaceIntegrate in ascending face order
+    int8_t stC = 0;
+    if (work) stC = u.status[c];
+    if (kTile) {
+        sWork[tid] = interior && work;
+        if (!__syncthreads_or(work)) return;
+        // each interior cell's +x, +y, +z fluxes (zero next to an empty cell)
+        if (interior && work) {
+#pragma unroll 1
+            for (int d = 0; d < 3; ++d) {
+                double q;
+                const int f = k0 + d;
+                sDv[d][tid] = faceDVf(m, u, f, true, c + m.latNb[3 + d], ac, stC, q);
+                u.alphaPhi[f] = q;
+            }
+        } else if (!work) {
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j)
-                if (sl[j].x != -2) add(sl[j].y);
-            for (int k = k0 + kBatch; k < k1; ++k) add(m.cSlot[k].y);
-            // the divisions through correctly rounded reciprocals (1/V per
-            // cell, 1/dt and 1/(1/dt) per step): the same quotients
-            const double ivf = divByRecip(sum, m.V[c], m.rV[c]);
-            double num = ao * rDeltaT;
-            if (Su) num = num + Su[c];
-            num = num - ivf * rDeltaT;
-            const double an = Sp ? num / (rDeltaT - Sp[c]) : divByRecip(num, rDeltaT, rrDeltaT);
-            aNew[c] = an;
-            // cells outside [-aTol, 1 + aTol] are the bounding candidates; the
-            // count of them decides limitFlux's loop (advectionTemplates.C:146)
-            // (on the bits: an < -aTol or an > 1 + aTol, NaN neither)
-            const double aTol = 100.0 * kSMALL;
-            const long long ba = bitsOf(an);
-            const long long mag = ba & 0x7fffffffffffffffLL;
-            ov = mag <= 0x7ff0000000000000LL && (ba < 0 ? mag > bitsOf(aTol) : ba > bitsOf(1.0 + aTol));
-            // only cells of the bounding set (mixed cells and their face
-            // neighbours, advection.C:54-82) are listed; every overshooting
-            // cell is counted
-            if (ov) {
-                inSet = status[c] != kStNotMixed;
-#pragma unroll
-                for (int j = 0; j < kBatch; ++j) inSet = inSet || (sl[j].x >= 0 && status[sl[j].x] != kStNotMixed);
-                for (int k = k0 + kBatch; k < k1 && !inSet; ++k) {
-                    const int nb = m.cSlot[k].x;
-                    inSet = nb >= 0 && status[nb] != kStNotMixed;
-                }
+            for (int d = 0; d < 3; ++d) sDv[d][tid] = 0.0;
+        }
+        // the fluxes through the tile's low sides, a thread each
+        if (tid < kHz + kHy + kHx) {
+            int src, slot;  // the cell of the tile and the slot of its face
+            if (tid < kHz) {
+                src = tid;
+                slot = 0;
+            } else if (tid < kHz + kHy) {
+                const int t = tid - kHz;
+                src = t % kDx + t / kDx * (TX * TY);
+                slot = 1;
+            } else {
+                src = (tid - kHz - kHy) * TX;
+                slot = 2;
+            }
+            if (sWork[src]) {
+                const int ci = blockIdx.x * TX + src % kDx, cj = blockIdx.y * TY + src / kDx % kDy,
+                          ck = blockIdx.z * TZ + src / (kDx * kDy);
+                const int cc = ci + m.latNx * (cj + m.latNy * ck);
+                const int f = latticeBase(cc, ci, cj, ck, ci + m.latNx * cj, m.latNx, m.latNy) + m.latFace[slot];
+                double q;
+                sLow[tid] = faceDVf(m, u, f, false, cc + m.latNb[slot], u.aCur[cc], u.status[cc], q);
+            }
+        }
+    }
+    if (work && !interior) {
+#pragma unroll 1
+        for (int q = k0; q < k1; ++q) {
+            const int2 s = m.cSlot[q];
+            const bool own = s.y >= 0;
+            const int f = s.y & 0x7fffffff;
+            double ap;
+            const double dv = faceDVf(m, u, f, own, s.x, ac, stC, ap);
+            if (own) {
+                u.alphaPhi[f] = ap;
+                sum += dv;
+                if (kTile && s.x >= 0) sDv[s.x == c + 1 ? 0 : (s.x == c + m.latNx ? 1 : 2)][tid] = dv;
+            } else {
+                sum -= dv;
+            }
+        }
+    }
+    if (kTile) {
+        __syncthreads();
+        if (work && interior) {
+            sum -= lk == 0 ? sLow[li + TX * lj] : sDv[2][tid - TX * TY];
+            sum -= lj == 0 ? sLow[kHz + li + TX * lk] : sDv[1][tid - TX];
+            sum -= li == 0 ? sLow[kHz + kHy + lj + TY * lk] : sDv[0][tid - 1];
+            sum += sDv[0][tid];
+            sum += sDv[1][tid];
+            sum += sDv[2][tid];
+        }
+    }
+    if (work) {
+        // the divisions through correctly rounded reciprocals (1/V per
+        // cell, 1/dt and 1/(1/dt) per step): the same quotients
+        const double ivf = divByRecip(sum, m.V[c], m.rV[c]);
+        double num = ao * u.rDeltaT;
+        if (u.Su) num = num + u.Su[c];
+        num = num - ivf * u.rDeltaT;
+        const double an = u.Sp ? num / (u.rDeltaT - u.Sp[c]) : divByRecip(num, u.rDeltaT, u.rrDeltaT);
+        u.aNew[c] = an;
+        // cells outside [-aTol, 1 + aTol] are the bounding candidates; the
+        // count of them decides limitFlux's loop (advectionTemplates.C:146)
+        // (on the bits: an < -aTol or an > 1 + aTol, NaN neither)
+        const double aTol = 100.0 * kSMALL;
+        const long long ba = bitsOf(an);
+        const long long mag = ba & 0x7fffffffffffffffLL;
+        ov = mag <= 0x7ff0000000000000LL && (ba < 0 ? mag > bitsOf(aTol) : ba > bitsOf(1.0 + aTol));
+        // only cells of the bounding set (mixed cells and their face
+        // neighbours, advection.C:54-82) are listed; every overshooting
+        // cell is counted
+        if (ov) {
+            inSet = stC != kStNotMixed;
+            const int nf = interior ? 6 : k1 - k0;
+            for (int q = 0; q < nf && !inSet; ++q) {
+                const int nb = interior ? c + m.latNb[q] : m.cSlot[k0 + q].x;
+                inSet = nb >= 0 && u.status[nb] != kStNotMixed;
             }
         }
     }
     const unsigned ball = __ballot_sync(0xffffffffu, ov);
     if (ball) {
         const int lane = threadIdx.x & 31;
-        if (lane == 0) atomicAdd(ovCount, __popc(ball));  // [0] all overshooting cells
+        if (lane == 0) atomicAdd(u.ovCount, __popc(ball));  // [0] all overshooting cells
         const unsigned sball = __ballot_sync(0xffffffffu, inSet);
         int base = 0;
-        if (lane == 0 && sball) base = atomicAdd(ovCount + 1, __popc(sball));  // [1] listed cells
+        if (lane == 0 && sball) base = atomicAdd(u.ovCount + 1, __popc(sball));  // [1] listed cells
         base = __shfl_sync(0xffffffffu, base, 0);
         const int p = base + __popc(sball & ((1u << lane) - 1u));
-        if (inSet && p < ovCap) ovList[p] = c;
+        if (inSet && p < u.ovCap) u.ovList[p] = c;
     }
 }
 
@@ -456,10 +596,24 @@ void launchInterfaceFaces(const StepArgs& a, cudaStream_t st) {
                                                             a.dt, a.dvfI, a.cutMask);
 }
 
+template <int TX, int TY, int TZ>
+static void launchUpdateTiles(const StepArgs& a, const UpdateArgs& u, cudaStream_t st) {
+    constexpr int kThreads = TX * TY * TZ;
+    static_assert(TX * TY + TX * TZ + TY * TZ <= kThreads, "at most one low side per thread");
+    const dim3 grid((a.m.latNx + TX - 1) / TX, (a.m.latNy + TY - 1) / TY, (a.m.latNz + TZ - 1) / TZ);
+    kUpdate<TX, TY, TZ><<<grid, kThreads, 0, st>>>(a.m, u);
+}
+
 void launchUpdate(const StepArgs& a, cudaStream_t st) {
-    const int nb = (a.m.nc + 255) / 256;
-    kUpdate<<<nb, 256, 0, st>>>(a.m, a.phi, a.aCur, a.aOld, a.aNew, a.status, a.dvfI, a.alphaB, a.Sp, a.Su, a.dt,
-                                a.rDeltaT, a.rrDeltaT, a.alphaPhi, a.ovList, a.ovCount, a.ovCap);
+    const UpdateArgs u{a.phi, a.aCur, a.aOld, a.aNew, a.status, a.dvfI, a.alphaB, a.Sp, a.Su, a.dt, a.rDeltaT,
+                       a.rrDeltaT, a.alphaPhi, a.ovList, a.ovCount, a.ovCap};
+    // every lattice whose tiles fit a grid (the other two dimensions of a
+    // grid end at 65,535)
+    if (a.m.latNx && (a.m.latNy + 3) / 4 <= 65535 && (a.m.latNz + 3) / 4 <= 65535) {
+        launchUpdateTiles<8, 4, 4>(a, u, st);
+        return;
+    }
+    kUpdate<0, 0, 0><<<(a.m.nc + 255) / 256, 256, 0, st>>>(a.m, u);
 }
 
 void launchBruteForce(const StepArgs& a, cudaStream_t st) {

@@ -541,6 +541,11 @@ int uploadMesh(simplic_handle* h, const simplic_mesh_desc* d, const HostMesh& hm
                 m.latNz = nz;
                 m.latDivLayer = dLayer;
                 m.latDivNx = dNx;
+                const int layer = nx * ny;
+                const int nbOff[6] = {-layer, -nx, -1, 1, nx, layer};
+                const int faceOff[6] = {2 - (3 * layer - nx - ny), 1 - (3 * nx - 1), -3, 0, 1, 2};
+                std::copy(nbOff, nbOff + 6, m.latNb);
+                std::copy(faceOff, faceOff + 6, m.latFace);
             }
         }
     }

@@ -273,6 +273,9 @@ struct DevMesh {
     int32_t latNx, latNy, latNz;  // a single-block lattice (cell i + nx (j + ny k), internal
                                   // faces by owner, +x +y +z): the slot records of every
                                   // interior cell follow from latticeSlots; else 0
+    int32_t latNb[6], latFace[6];  // of an interior lattice cell c: the cell across slot k is
+                             // c + latNb[k], its face latticeBase(c) + latFace[k] (slots 0-2
+                             // on the neighbour side)
     const double* pts;       // [3 np]
     const int32_t* fOff;     // [nf+1]
     const int32_t* fPts;     // face point lists, stored order
@@ -377,18 +380,21 @@ __device__ __forceinline__ int stencilOf(const DevMesh& m, int c, const int32_t*
 // false for a boundary cell.  For an interior cell every owner involved
 // owns all three of its faces, so the owners c - 1, c - nx, c - nx ny start
 // 3, 3 nx - 1 and 3 nx ny - nx - ny faces before c.
+// internal faces owned by the cells before an interior cell c = i + nx (j +
+// ny k), p = i + nx j (faces are ordered by owner, each owner's +x, +y, +z in
+// turn): +x faces, nx - 1 per earlier row plus one per earlier cell of c's
+// row; +y faces, nx (ny - 1) per earlier layer plus one per earlier cell of
+// c's layer; +z faces, one per earlier cell (every earlier cell in c's row /
+// layer / the mesh owns that face because c is interior)
+__host__ __device__ __forceinline__ int latticeBase(int c, int i, int j, int k, int p, int nx, int ny) {
+    return (j + ny * k) * (nx - 1) + i + k * nx * (ny - 1) + p + c;
+}
 // The records of cell c = i + nx (j + ny k), p = i + nx j, when it is interior.
 __host__ __device__ __forceinline__ bool latticeSlotsAt(int c, int i, int j, int k, int p, int nx, int ny, int nz,
                                                         int2 (&sl)[6]) {
     const int layer = nx * ny;
     if (i == 0 || j == 0 || k == 0 || i == nx - 1 || j == ny - 1 || k == nz - 1) return false;
-    // internal faces owned by the cells before c (faces are ordered by
-    // owner, each owner's +x, +y, +z in turn): +x faces, nx - 1 per earlier
-    // row plus one per earlier cell of c's row; +y faces, nx (ny - 1) per
-    // earlier layer plus one per earlier cell of c's layer; +z faces, one
-    // per earlier cell (every earlier cell in c's row / layer / the mesh
-    // owns that face because c is interior)
-    const int b = (j + ny * k) * (nx - 1) + i + k * nx * (ny - 1) + p + c;
+    const int b = latticeBase(c, i, j, k, p, nx, ny);
     const unsigned side = 0x80000000u;
     sl[0] = make_int2(c - layer, int(unsigned(b - (3 * layer - nx - ny) + 2) | side));
     sl[1] = make_int2(c - nx, int(unsigned(b - (3 * nx - 1) + 1) | side));

@@ -14,17 +14,26 @@
 //     the bounding set; their dependencies are found through per-cell stamps,
 //     no sorting;
 //   * dataflow: everything of a cell's loop that reads no correction is
-//     computed for all overshooting cells at once; a cell then runs as soon
-//     as the earlier neighbours it waits for have stored the corrections on
-//     the faces it shares with them -- the one that completes it runs it
-//     next in the same warp (chains run through in one warp) and a ready
-//     queue feeds the idle warps -- and the corrected-face lists are built
+//     computed for all overshooting cells at once; a cell then starts as soon
+//     as the earlier neighbours it waits for have started -- the last of them
+//     runs it next in the same warp (chains run through in one warp) and a
+//     queue feeds the idle warps -- and polls for the corrections on the
+//     faces it shares with them; the corrected-face lists are built
 //     afterwards, off the dependency chains;
 //   * corrections are applied per target cell in the reference's list order
 //     (key = cell * 32 + position among the cell's first-iteration faces);
 //   * the pass test max(alpha) - 1 > aTol || min(alpha) < -aTol is exactly
 //     "some cell of the mesh overshoots": an exact counter of overshooting
 //     cells replaces the global min / max.
+// What bounds it is latency: dependent L2 accesses (0.4 us each), the FP64
+// chain of a cell's loop (0.3 us) along chains of up to 70 cells a pass, and
+// four barriers a pass (2-3 us each).  One GB300, kernel time before the
+// records came ahead through shared memory, cells were handed over inside a
+// block and the other phases took 8 lanes per cell -> after: 256^3 with 6,900
+// overshooting cells in the first of three passes 0.81 -> 0.47 ms (dependency
+// phases 0.64 -> 0.35), 128^3 (7,500) 0.32 -> 0.20 ms (0.14 -> 0.09), 96^3
+// warped hexahedra (5,300) 0.71 -> 0.40 ms, 45^3 x 6 tetrahedra (3,400) 0.19
+// -> 0.15 ms, 33^3 (31) 0.086 -> 0.078 ms.
 // Blocks meet at a grid barrier whose wait is bounded (a timeout sets an
 // error bit and ends the blocks that see it); every loop and every wait of
 // the dependency phase is bounded too, and no block returns after the first
@@ -42,7 +51,11 @@ namespace {
 
 constexpr double kATol = 100.0 * kSMALL;  // advectionTemplates.C:125,228
 
-__device__ __forceinline__ bool overshoots(double a) { return a < -kATol || a > 1.0 + kATol; }
+// a < -aTol || a > 1 + aTol on the bits (a NaN neither)
+__device__ __forceinline__ bool overshoots(double a) {
+    const long long b = bitsOf(a), mag = b & 0x7fffffffffffffffLL;
+    return mag <= 0x7ff0000000000000LL && (b < 0 ? mag > bitsOf(kATol) : b > bitsOf(1.0 + kATol));
+}
 __device__ __forceinline__ unsigned long long globalNs() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -187,7 +200,7 @@ struct BoundLane {
     bool pass0;              // passing in the first iteration when no correction arrives
     double maxExtra0, through0;
 };
-struct BoundCellConst {
+struct alignas(16) BoundCellConst {
     double Vi, rVi;        // cell volume, 1 / V
     double ov0, fluid0;    // alphaOvershoot and fluid of the first iteration
     double num1;           // alpha.oldTime * rDeltaT (+ Su) - netFlux(dVf) / V * rDeltaT
@@ -197,8 +210,38 @@ struct BoundCellConst {
     int eNum1, eRden;      // exponent fields of num1, rden
     unsigned pm0, ownMask; // first-iteration passing faces without corrections; owner-side faces
     int nfc, pad;          // faces of the cell
+    double pad2;           // to 16-byte multiples
 };
 static_assert(sizeof(BoundCellConst) == kBoundCellConstBytes, "per-candidate constant record size");
+// A face of an overshooting candidate as the dependency phase reads it.
+struct alignas(16) BoundSlot {
+    double dv, phdt, max0, thr0;  // BoundLane's dv, phdt, maxExtra0, through0
+    int F, succ;                  // face; later overshooting candidate across it when it is downwind, or -1
+    int flags, pad;               // kSlot* bits
+};
+static_assert(sizeof(BoundSlot) == kBoundSlotBytes, "face slot size");
+__device__ __forceinline__ uint8_t* recordOf(const BoundBuffers& s, int i) { return s.rec + size_t(i) * s.recBytes; }
+__device__ __forceinline__ BoundSlot* slotsOf(const BoundBuffers& s, int i) {
+    return reinterpret_cast<BoundSlot*>(recordOf(s, i) + kBoundCellConstBytes);
+}
+// Shared memory a warp has for records: four of a hexahedron, one of any cell.
+constexpr int kWarpRecordBytes = 2048;
+static_assert(boundRecordBytes(6) * 4 <= kWarpRecordBytes && boundRecordBytes(kMaxCellFaces) <= kWarpRecordBytes,
+              "record buffers");
+// A record into the warp's shared buffer, asynchronously; fetchWait makes it
+// visible to the warp.
+__device__ __forceinline__ void fetchRecord(uint8_t* buf, const BoundBuffers& s, int i, int lane) {
+    const uint8_t* r = recordOf(s, i);
+    for (int o = 16 * lane; o < s.recBytes; o += 512)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(buf + o))),
+                     "l"(r + o)
+                     : "memory");
+}
+__device__ __forceinline__ void fetchWait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+}
 
 // face-slot flags of an overshooting candidate
 enum : uint8_t { kSlotOn = 1, kSlotOwn = 2, kSlotDown = 4, kSlotPhPos = 8, kSlotPass0 = 16, kSlotDep = 32 };
@@ -288,20 +331,23 @@ __device__ __forceinline__ void boundCellPrep(int c, int nfc, int nmax, int base
 // the only case in which it can write one; zero otherwise (a later
 // neighbour writes only after this cell in the reference's order, an
 // inactive one writes nothing).  Returns this lane's final correction;
-// pmFirst gets the faces that pass in the first iteration.
+// pmFirst gets the faces that pass in the first iteration; ahead() is called
+// once, in the first iteration, for work that the loop's latency can hide.
+template <class Ahead>
 __device__ __forceinline__ double boundCellLoop(bool hasDep, double cr0, const BoundLane& L,
-                                                const BoundCellConst& kc, const StepArgs& a, int lane,
-                                                unsigned& pmFirst) {
+                                                const BoundCellConst& kc, const StepArgs& a, unsigned& pmFirst,
+                                                Ahead&& ahead) {
     constexpr unsigned kAll = 0xffffffffu;
     double cr = cr0;
     double ov = kc.ov0, fluid = kc.fluid0;
-    int nPass = 1;
     pmFirst = 0;
-    for (int iter = 0; iter < 10; ++iter) {
-        if (absLess(ov, kATol) || nPass == 0) break;
+    unsigned sumOf = 0;            // the faces dVftot was last summed over
+    double dVftot = 0.0, rTot = 0.0;
+    // one iteration; false ends the loop
+    const auto step = [&](bool first, bool last) -> bool {
         bool pass = false;
         double pmax = 0.0;
-        if (iter == 0 && !hasDep) {
+        if (first && !hasDep) {
             pass = L.pass0;
             pmax = L.maxExtra0;
         } else if (L.down) {
@@ -316,24 +362,33 @@ __device__ __forceinline__ double boundCellLoop(bool hasDep, double cr0, const B
         }
         const unsigned pm = __ballot_sync(kAll, pass);
         double through = 0.0;
-        if (iter == 0 && pm == kc.pm0) {
+        if (first && pm == kc.pm0) {
             through = L.through0;  // the same faces, so the same dVftot
         } else {
-            double dVftot = 0.0;
-            for (unsigned mm = pm; mm; mm &= mm - 1u) dVftot += __shfl_sync(kAll, L.aPhdt, __ffs(mm) - 1);
-            if (pass) through = fabs(fluid) * L.aPhdt / dVftot;
+            if (pm != sumOf) {
+                dVftot = 0.0;
+                for (unsigned mm = pm; mm; mm &= mm - 1u) dVftot += __shfl_sync(kAll, L.aPhdt, __ffs(mm) - 1);
+                sumOf = pm;
+                rTot = 1.0 / dVftot;
+            }
+            if (pass) through = divByRecip(fabs(fluid) * L.aPhdt, dVftot, rTot);
         }
         int passInc = 0;
         if (pass) {
-            passInc = geZero(pmax - through) ? 1 : 0;  // pos0(maxExtra - through)
+            // pos0(maxExtra - through) of two values >= 0, on the bits (a NaN never)
+            passInc = bitsOf(pmax) >= bitsOf(through) && bitsOf(pmax) <= 0x7ff0000000000000LL &&
+                      (bitsOf(pmax) < 0x7ff0000000000000LL || bitsOf(through) < 0x7ff0000000000000LL);
             through = minNonNeg(through, pmax);
             // sign(phi) sign(fluid) through is +-through exactly
             cr = cr + ((L.phPos == geZero(fluid)) ? through : -through);
         }
-        nPass = __reduce_add_sync(kAll, passInc);
-        if (iter == 0) pmFirst = pm;
+        const int nPass = __popc(__ballot_sync(kAll, passInc));
+        if (first) {
+            pmFirst = pm;
+            ahead();
+        }
         // the next test ends the loop without reading alpha1New
-        if (nPass == 0 || iter == 9) break;
+        if (nPass == 0 || last) return false;
         double nf2 = 0.0;  // netFlux(c, dVfcorrectionValues), face order
         const unsigned nz = __ballot_sync(kAll, L.on && !isZero(cr));
         for (unsigned mm = nz; mm; mm &= mm - 1u) {
@@ -351,42 +406,57 @@ __device__ __forceinline__ double boundCellLoop(bool hasDep, double cr0, const B
         const double a1 = (kc.num1 - t2) * kc.rden;
         const long long b1 = bitsOf(a1);
         const bool inWindow = b1 >= 0 ? b1 < bitsOf(kUnitHi) : (b1 & 0x7fffffffffffffffLL) < bitsOf(kHalfATol);
-        if (inWindow && max(kc.eNum1, expField(t2)) + kc.eRden <= 2045) break;
+        if (inWindow && max(kc.eNum1, expField(t2)) + kc.eRden <= 2045) return false;
         double num = kc.num1;
         num = num - divByRecip(nf2, kc.Vi, kc.rVi) * a.rDeltaT;
         const double a1New = divByRecip(num, kc.den, kc.rden);
-        ov = pos0(a1New - 1.0) * (a1New - 1.0) + neg0(a1New) * a1New;
+        // pos0(a1New - 1) (a1New - 1) + neg0(a1New) a1New up to the sign of a zero (NaN stays)
+        const long long bn = bitsOf(a1New);
+        if (bn >= bitsOf(1.0))
+            ov = a1New - 1.0;
+        else
+            ov = ltZero(a1New) || (bn & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL ? a1New : 0.0;
         fluid = ov * kc.Vi;
+        return !absLess(ov, kATol);
+    };
+    if (absLess(ov, kATol)) {
+        ahead();
+        return cr;
     }
-    (void)lane;
+    // (the first iteration apart: nine in ten cells have no other, and what
+    // ahead() waits for is not waited for before it)
+    if (step(true, false))
+        for (int iter = 1; iter < 10 && step(false, iter == 9); ++iter) {
+        }
     return cr;
 }
 
-// After the dependency phase, for one overshooting cell (a warp, lane k on
-// face k): the faces that passed in its first iteration join the list of
-// corrected faces (key cell * 32 + position, the reference's list order)
-// with their new dVf, and the cells on both sides become targets of the
-// pass.  No later cell changes the correction of such a face, as a face is
-// downwind for one side only.
-__device__ void boundCellLists(int i, const DevMesh& m, const StepArgs& a, const BoundBuffers& s, int lane,
+// After the dependency phase, for the overshooting cells of a warp (a group
+// of lanes each, lane gl on the cell's gl-th face; i < 0: no cell): the faces
+// that passed in a cell's first iteration join the list of corrected faces
+// (key cell * 32 + position, the reference's list order) with their new dVf,
+// and the cells on both sides become targets of the pass.  No later cell
+// changes the correction of such a face, as a face is downwind for one side
+// only.
+__device__ void boundCellLists(int i, int gl, const DevMesh& m, const StepArgs& a, const BoundBuffers& s, int lane,
                                int pass, int passStamp, int stamp) {
     constexpr unsigned kAll = 0xffffffffu;
     const unsigned below = (1u << lane) - 1u;
-    const int c = s.cand[i];
-    const unsigned pmFirst = s.candPm[i];
-    const bool first = (pmFirst >> lane) & 1u;
+    const int c = i >= 0 ? s.cand[i] : 0;
+    const unsigned pmFirst = i >= 0 ? s.candPm[i] : 0u;
+    const bool first = (pmFirst >> gl) & 1u;
     int f = 0, t0 = -1, t1 = -1, c0 = passStamp, c1 = passStamp;
     bool fresh = false;
     if (first) {
-        f = s.slotF[size_t(i) * m.maxCellFaces + lane];
+        f = slotsOf(s, i)[gl].F;
         const double cr = s.corr[f];
         t0 = m.own[f];
         t1 = f < m.nfi ? m.nei[f] : -1;
         c0 = atomicExch(s.cellClaim + t0, passStamp);
         if (t1 >= 0) c1 = atomicExch(s.cellClaim + t1, passStamp);
-        s.faceKey[f] = unsigned(c) * 32u + unsigned(__popc(pmFirst & below));
+        s.faceKey[f] = unsigned(c) * 32u + unsigned(__popc(pmFirst & ((1u << gl) - 1u)));
         s.faceStamp[f] = passStamp;
-        const double nv = curDVf(m, f, a.phi, a.aCur, a.status, a.dvfI, a.alphaB, a.dt, s, stamp) + cr;
+        const double nv = slotsOf(s, i)[gl].dv + cr;  // dv: the dVf the pass started from
         fresh = s.modStamp[f] != stamp;
         s.dvfMod[f] = nv;
         s.modStamp[f] = stamp;
@@ -417,7 +487,7 @@ __device__ void boundCellLists(int i, const DevMesh& m, const StepArgs& a, const
     }
 }
 
-// ready-queue entries carry the pass stamp, so stale ones never match
+// queue entries carry the pass stamp, so stale ones never match
 __device__ __forceinline__ void stQueue(unsigned long long* p, int passStamp, int i) {
     const unsigned long long v = (static_cast<unsigned long long>(unsigned(passStamp)) << 32) | unsigned(i);
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -438,7 +508,20 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
     const int gw = tid >> 5, nw = nth >> 5;
     const int stamp = s.stamp;  // step stamp
     unsigned barK = 0;          // grid barriers passed
+    // Outside the dependency phase a cell takes a group of lanes, lane gl of it
+    // on the cell's gl-th face: 8, 16 or 32 lanes as the mesh's cells have
+    // faces.  These phases are latency and FP64 warp instructions, both per
+    // warp, so more cells to a warp are as many times fewer of them.
+    const int gsz = m.maxCellFaces <= 8 ? 8 : (m.maxCellFaces <= 16 ? 16 : 32);
+    const int per = 32 / gsz, gl = lane & (gsz - 1), base = lane - gl;
+    const unsigned gbits = gsz == 32 ? 0xffffffffu : (1u << gsz) - 1u;
     const bool clock0 = tid == 0;  // block 0 keeps the time profile
+    __shared__ __align__(16) uint8_t recBuf[8][kWarpRecordBytes];  // per warp: records of the cells it may run next
+    // a warp that waits for a cell from its own block: kMailIdle, or the cell
+    // another warp gave it; kMailBusy otherwise
+    __shared__ int mail[8];
+    __shared__ int allRun;
+    constexpr int kMailIdle = -1, kMailBusy = -2;
     const unsigned long long tStart = clock0 ? globalNs() : 0ull;
     unsigned long long tDep = 0ull;
     // Decisions before the first barrier read values no block modifies.
@@ -468,29 +551,23 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
         const int passStamp = stamp * kMaxBoundPasses + pass + 1;
         const int nCand = ldVol(s.ctl + kCtlCand);
         if (tid == 0) s.info[0] = pass + 1;
-        // 2. the overshooting candidates (a half-warp or a warp per candidate,
-        //    lane k of it on the cell's k-th face in cells() order): per face
-        //    the dVf the pass
+        // 2. the overshooting candidates (a group of lanes each, on the cell's
+        //    faces in cells() order): per face the dVf the pass
         //    starts from (final here: earlier passes are complete), the
         //    earlier overshooting cell it waits for (when the face is
         //    downwind for that cell, the only case in which it writes a
-        //    correction there) and the later one it releases; then the loop's
+        //    correction there) and the later one that waits for it; then the loop's
         //    parts that read no correction.  Cells that wait for nobody go to
-        //    the ready queue.
+        //    the front of the queue.
         {
-            // two candidates per warp (a half-warp each) while every cell has
-            // at most 16 faces, else one
-            const bool wide = m.maxCellFaces > 16;
-            const int per = wide ? 1 : 2;
-            const int base = wide ? 0 : (lane & 16), gl = lane - base;
-            const unsigned gbits = wide ? 0xffffffffu : 0xffffu;
             for (int r0 = gw * per; r0 < nCand; r0 += nw * per) {
-                const int i = r0 + (base >> 4);
+                const int i = r0 + lane / gsz;
                 const bool valid = i < nCand;
-                const int c = valid ? s.cand[i] : s.cand[r0];
+                const int c = s.cand[valid ? i : r0];
                 const bool act = valid && overshoots(a.aNew[c]);
                 if (!__any_sync(kAll, act)) continue;  // the same on every lane
-                const int k0 = m.cOff[c], nfc = act ? m.cOff[c + 1] - k0 : 0;
+                const int k0 = m.uniformFaces ? c * m.uniformFaces : m.cOff[c];
+                const int nfc = !act ? 0 : (m.uniformFaces ? m.uniformFaces : m.cOff[c + 1] - k0);
                 const int nmax = __reduce_max_sync(kAll, nfc);
                 int Fs = 0, succ = -1;
                 bool dep = false;
@@ -517,23 +594,24 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
                 boundCellPrep(c, nfc, nmax, base, gbits, Fs, ph, dv, m, a, gl, L, k);
                 const unsigned depMask = (__ballot_sync(kAll, dep) >> base) & gbits;
                 if (L.on) {
-                    const size_t sl = size_t(i) * m.maxCellFaces + gl;
-                    s.slotF[sl] = L.F;
-                    s.slotFlags[sl] = uint8_t(kSlotOn | (L.own ? kSlotOwn : 0) | (L.down ? kSlotDown : 0) |
-                                              (L.phPos ? kSlotPhPos : 0) | (L.pass0 ? kSlotPass0 : 0) |
-                                              (dep ? kSlotDep : 0));
-                    s.slotSucc[sl] = succ;
-                    s.slotDv[sl] = L.dv;
-                    s.slotPhdt[sl] = L.phdt;
-                    s.slotMax0[sl] = L.maxExtra0;
-                    s.slotThr0[sl] = L.through0;
+                    BoundSlot v;
+                    v.dv = L.dv;
+                    v.phdt = L.phdt;
+                    v.max0 = L.maxExtra0;
+                    v.thr0 = L.through0;
+                    v.F = L.F;
+                    v.succ = succ;
+                    v.flags = kSlotOn | (L.own ? kSlotOwn : 0) | (L.down ? kSlotDown : 0) |
+                              (L.phPos ? kSlotPhPos : 0) | (L.pass0 ? kSlotPass0 : 0) | (dep ? kSlotDep : 0);
+                    v.pad = 0;
+                    slotsOf(s, i)[gl] = v;
                 }
                 if (gl == 0 && act) {
-                    reinterpret_cast<BoundCellConst*>(s.candK)[i] = k;
-                    s.candDepN[i] = __popc(depMask);
+                    k.pad2 = 0.0;
+                    *reinterpret_cast<BoundCellConst*>(recordOf(s, i)) = k;
                     s.candPending[i] = __popc(depMask);
                     s.actList[atomicAdd(s.ctl + kCtlActive0 + pass, 1)] = i;
-                    if (depMask == 0) stQueue(s.readyQ + atomicAdd(s.ctl + kCtlQTail0 + pass, 1), passStamp, i);
+                    if (depMask == 0) stQueue(s.readyQ + atomicAdd(s.ctl + kCtlFree0 + pass, 1), passStamp, i);
                 }
             }
         }
@@ -541,121 +619,202 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
         const int nAct = ldVol(s.ctl + kCtlActive0 + pass);
         // no listed cell overshoots: this and every later pass change nothing
         if (nAct == 0) break;
-        // 3. dependencies as dataflow.  A cell runs once every earlier
-        //    overshooting neighbour it waits for has stored its corrections:
-        //    the neighbour that completes it (the last one to decrement its
-        //    count, or its only one) runs it next in the same warp, so a chain
-        //    runs through in one warp; the others it completes go to the ready
-        //    queue, from which idle warps take cells until all are done.  The
-        //    correction values are their own flags (a face holds the pending
-        //    NaN until the earlier cell stores it; a 64-bit store is single-
-        //    copy atomic), so a released cell needs no fence.  Every wait is
-        //    bounded: one that runs out sets the timeout bit and the warp
-        //    stops; the others then stop at their own limits.
+        // 3. dependencies as dataflow.  A cell may start once every earlier
+        //    overshooting neighbour it waits for has started: the neighbour
+        //    that starts last (by an atomic count) runs it next in the same
+        //    warp, so a chain runs through in one warp; the others it releases
+        //    go to the queue.  The correction values are their own flags (a
+        //    face holds the pending NaN until the earlier cell stores it; a
+        //    64-bit store is single-copy atomic), so a cell polls for what a
+        //    neighbour in another warp is still computing -- that warp waits
+        //    for nothing but cells that have started before it -- and takes
+        //    the value of the cell its own warp has just run from registers.
+        //    What a link of a chain costs is memory latency (about 0.4 us per
+        //    dependent access; a cell's loop itself takes 0.3 us), so: the
+        //    count goes ahead of the loop; the records of the cells that wait
+        //    for this one come into shared memory meanwhile; and a released
+        //    cell goes to a waiting warp of the same block through shared
+        //    memory, to the queue (two atomics and two polls later in another
+        //    block) only when there is none.
+        //    Every wait is bounded: one that runs out sets the timeout bit and
+        //    the warp stops; the others then stop at their own limits.
         const unsigned long long td0 = clock0 ? globalNs() : 0ull;
         {
-            int longest = 0;
+            const int nFree = ldVol(s.ctl + kCtlFree0 + pass);
+            const int wl = threadIdx.x >> 5;
+            const bool taker = wl < 2;  // these two wait for the queue, the other six for cells of the block
+            uint8_t* const bufs = recBuf[wl];
+            const int nBuf = kWarpRecordBytes / s.recBytes;
+            if (lane == 0) mail[wl] = kMailBusy;
+            if (threadIdx.x == 0) allRun = 0;
+            __syncthreads();
+            volatile int* const vMail = mail;
+            int longest = 0, starts = 0, h = gw;  // the first free cell without an atomic
             bool failed = false;
-            while (!failed) {
-                int h = 0;
-                if (lane == 0) h = atomicAdd(s.ctl + kCtlQHead0 + pass, 1);
-                h = __shfl_sync(kAll, h, 0);
-                if (h >= nAct) break;  // more takers than cells: nothing left for this warp
+            for (;;) {
                 int i = -1;
-                if (lane == 0) {
+                if (h < nFree) {
+                    i = int(unsigned(s.readyQ[h]));
+                } else if (taker) {
+                    if (lane == 0) {
+                        const int e = atomicAdd(s.ctl + kCtlQHead0 + pass, 1);
+                        for (long long spin = 0;; ++spin) {
+                            const unsigned long long v = e < nAct ? ldQueue(s.readyQ + (s.candCap - 1 - e)) : 0ull;
+                            if (unsigned(v >> 32) == unsigned(passStamp)) {
+                                i = int(unsigned(v));
+                                break;
+                            }
+                            if (ldVol(s.ctl + kCtlDone0 + pass) >= nAct) break;  // all done: entry e never comes
+                            if (spin >= s.spinLimit) {
+                                atomicOr(a.err, (uint32_t)kErrBarrierTimeout);
+                                i = -3;
+                                break;
+                            }
+                            __nanosleep(64);
+                        }
+                        if (i < 0) *(volatile int*)&allRun = 1;
+                    }
+                } else if (lane == 0) {
+                    vMail[wl] = kMailIdle;
                     for (long long spin = 0;; ++spin) {
-                        const unsigned long long e = ldQueue(s.readyQ + h);
-                        if (unsigned(e >> 32) == unsigned(passStamp)) {
-                            i = int(unsigned(e));
+                        const int v = vMail[wl];
+                        if (v >= 0) {
+                            i = v;
                             break;
                         }
-                        if (ldVol(s.ctl + kCtlDone0 + pass) >= nAct) break;  // all done: entry h never comes
-                        if (spin >= s.spinLimit) {
+                        // (every cell has run, or a taker gave up: no mail comes any more)
+                        if (*(volatile int*)&allRun) break;
+                        if (spin >= 4 * s.spinLimit) {
                             atomicOr(a.err, (uint32_t)kErrBarrierTimeout);
-                            i = -2;
                             break;
                         }
-                        __nanosleep(100);
+                        __nanosleep(32);
                     }
-                    if (i >= 0) atomicAdd(s.ctl + kCtlStarts0 + pass, 1);
+                    vMail[wl] = kMailBusy;
                 }
-                i = __shfl_sync(kAll, i, 0);
-                if (i == -2) failed = true;
+                if (h >= nFree) i = __shfl_sync(kAll, i, 0);
                 if (i < 0) break;
-                for (int hop = 0; i >= 0; ++hop) {
-                    const BoundCellConst k = reinterpret_cast<const BoundCellConst*>(s.candK)[i];
-                    BoundLane L;
-                    uint8_t fl = 0;
-                    int succ = -1;
-                    L.F = 0;
-                    L.dv = L.phdt = L.maxExtra0 = L.through0 = 0.0;
-                    if (lane < k.nfc) {
-                        const size_t sl = size_t(i) * m.maxCellFaces + lane;
-                        fl = s.slotFlags[sl];
-                        L.F = s.slotF[sl];
-                        succ = s.slotSucc[sl];
-                        L.dv = s.slotDv[sl];
-                        L.phdt = s.slotPhdt[sl];
-                        L.maxExtra0 = s.slotMax0[sl];
-                        L.through0 = s.slotThr0[sl];
+                ++starts;
+                int gotF = -1;  // the face whose correction this warp has just formed, and that
+                double gotCr = 0.0;
+                int ran = 0, at = 0;  // cells run; the buffer with the cell's record
+                fetchRecord(bufs, s, i, lane);
+                while (i >= 0) {
+                    fetchWait();
+                    const uint8_t* const rec = bufs + at * s.recBytes;
+                    const BoundCellConst k = *reinterpret_cast<const BoundCellConst*>(rec);
+                    BoundSlot v;
+                    v.flags = 0;
+                    v.F = 0;
+                    v.succ = -1;
+                    v.dv = v.phdt = v.max0 = v.thr0 = 0.0;
+                    if (lane < k.nfc) v = reinterpret_cast<const BoundSlot*>(rec + kBoundCellConstBytes)[lane];
+                    const int succ = v.succ;
+                    // count this cell as started for its successors, and fetch their records
+                    // (under a predicate in one instruction: a select after the atomic
+                    // would wait for it here)
+                    int left = 0;
+                    asm volatile(
+                        "{\n .reg .pred p;\n setp.ge.s32 p, %2, 0;\n @p atom.relaxed.gpu.global.add.s32 %0, [%1], -1;\n}"
+                        : "+r"(left)
+                        : "l"(s.candPending + (succ >= 0 ? succ : 0)), "r"(succ)
+                        : "memory");
+                    const unsigned sm = __ballot_sync(kAll, succ >= 0);  // (everybody has read the record)
+                    {
+                        int b = 0;
+                        for (unsigned mm = sm; mm && b < nBuf; mm &= mm - 1u, ++b)
+                            fetchRecord(bufs + b * s.recBytes, s, __shfl_sync(kAll, succ, __ffs(mm) - 1), lane);
                     }
-                    L.on = fl & kSlotOn;
-                    L.own = fl & kSlotOwn;
-                    L.down = fl & kSlotDown;
-                    L.phPos = fl & kSlotPhPos;
-                    L.pass0 = fl & kSlotPass0;
+                    BoundLane L;
+                    L.F = v.F;
+                    L.dv = v.dv;
+                    L.phdt = v.phdt;
+                    L.maxExtra0 = v.max0;
+                    L.through0 = v.thr0;
+                    L.on = v.flags & kSlotOn;
+                    L.own = v.flags & kSlotOwn;
+                    L.down = v.flags & kSlotDown;
+                    L.phPos = v.flags & kSlotPhPos;
+                    L.pass0 = v.flags & kSlotPass0;
                     L.aPhdt = fabs(L.phdt);
-                    const bool hasDep = fl & kSlotDep;
-                    // how many cells this lane's successor waits for (read
-                    // ahead; final since the candidates phase)
-                    const int sDepN = succ >= 0 ? s.candDepN[succ] : 0;
+                    const bool hasDep = v.flags & kSlotDep;
                     long long cv = 0;  // bits of +0
                     bool stuck = false;
                     if (hasDep) {
-                        for (long long spin = 0;; ++spin) {
-                            cv = ldRelaxed64(s.corr + L.F);
-                            if (cv != kCorrPending) break;
-                            if (spin >= s.spinLimit) {
-                                atomicOr(a.err, (uint32_t)kErrBarrierTimeout);
-                                stuck = true;
-                                break;
+                        if (L.F == gotF) {
+                            cv = bitsOf(gotCr);
+                        } else {
+                            for (long long spin = 0;; ++spin) {
+                                cv = ldRelaxed64(s.corr + L.F);
+                                if (cv != kCorrPending) break;
+                                if (spin >= s.spinLimit) {
+                                    atomicOr(a.err, (uint32_t)kErrBarrierTimeout);
+                                    stuck = true;
+                                    break;
+                                }
                             }
-                            __nanosleep(32);
                         }
                     }
                     if (__any_sync(kAll, stuck)) {
                         failed = true;
                         break;
                     }
-                    unsigned pmFirst = 0;
-                    const double cr = boundCellLoop(hasDep, __longlong_as_double(cv), L, k, a, lane, pmFirst);
+                    unsigned pmFirst = 0, rm = 0;
+                    double cr = boundCellLoop(hasDep, __longlong_as_double(cv), L, k, a, pmFirst, [&] {
+                        // the cells this one was the last to wait for
+                        rm = __ballot_sync(kAll, left == 1);
+                        // one is this warp's next; the others go to waiting warps of the block or the queue
+                        unsigned rest = rm & (rm - 1u);
+                        while (rest) {
+                            const int c = __shfl_sync(kAll, succ, __ffs(rest) - 1);
+                            rest &= rest - 1u;
+                            unsigned idle = __ballot_sync(kAll, lane < 8 && vMail[lane & 7] == kMailIdle);
+                            bool given = false;
+                            while (idle && !given) {
+                                int old = 0;
+                                if (lane == 0) old = atomicCAS(&mail[__ffs(idle) - 1], kMailIdle, c);
+                                given = __shfl_sync(kAll, old, 0) == kMailIdle;
+                                idle &= idle - 1u;
+                            }
+                            if (!given && lane == 0)
+                                stQueue(s.readyQ + (s.candCap - 1 - atomicAdd(s.ctl + kCtlQTail0 + pass, 1)), passStamp,
+                                        c);
+                        }
+                    });
+                    if (bitsOf(cr) == kCorrPending) cr = __longlong_as_double(0x7fffffffffffffffLL);
                     // only downwind faces can carry this cell's corrections, and
                     // each face is downwind for one side only: the face's one writer
-                    if (L.down)
-                        stRelaxed64(s.corr + L.F,
-                                    bitsOf(cr) == kCorrPending ? __longlong_as_double(0x7fffffffffffffffLL) : cr);
-                    if (lane == 0) {
-                        s.candPm[i] = pmFirst;
-                        atomicAdd(s.ctl + kCtlDone0 + pass, 1);
+                    if (L.down) stRelaxed64(s.corr + L.F, cr);
+                    if (lane == 0) s.candPm[i] = pmFirst;
+                    ++ran;
+                    i = -1;
+                    if (rm) {
+                        const int src = __ffs(rm) - 1;
+                        i = __shfl_sync(kAll, succ, src);
+                        gotF = __shfl_sync(kAll, L.F, src);
+                        gotCr = __shfl_sync(kAll, cr, src);
+                        at = __popc(sm & ((1u << src) - 1u));
+                        if (at >= nBuf) {  // no buffer was left for it
+                            fetchWait();
+                            at = 0;
+                            fetchRecord(bufs, s, i, lane);
+                        }
                     }
-                    __syncwarp();
-                    // release the later cells across the downwind faces
-                    const bool rel = succ >= 0 && (sDepN == 1 || atomicSub(s.candPending + succ, 1) == 1);
-                    const unsigned rm = __ballot_sync(kAll, rel);
-                    longest = max(longest, hop + 1);
-                    if (!rm) break;
-                    const unsigned rest = rm & (rm - 1u);
-                    if (rest) {
-                        int base = 0;
-                        if (lane == 0) base = atomicAdd(s.ctl + kCtlQTail0 + pass, __popc(rest));
-                        base = __shfl_sync(kAll, base, 0);
-                        if ((rest >> lane) & 1u)
-                            stQueue(s.readyQ + base + __popc(rest & ((1u << lane) - 1u)), passStamp, succ);
-                    }
-                    i = __shfl_sync(kAll, succ, __ffs(rm) - 1);
+                }
+                fetchWait();  // nothing is in flight when the buffers are filled again
+                longest = max(longest, ran);
+                if (lane == 0) atomicAdd(s.ctl + kCtlDone0 + pass, ran);
+                if (failed) break;
+                if (h < nFree) {
+                    if (lane == 0) h = nw + atomicAdd(s.ctl + kCtlFreeHead0 + pass, 1);
+                    h = __shfl_sync(kAll, h, 0);
                 }
             }
-            if (lane == 0 && longest > 0) atomicMax(s.info + 4, longest);
+            if (lane == 0 && failed) *(volatile int*)&allRun = 1;
+            if (lane == 0 && longest > 0) {
+                atomicMax(s.info + 4, longest);
+                atomicAdd(s.ctl + kCtlStarts0 + pass, starts);
+            }
         }
         if (!gridBarrier(s, a.err, barK)) return;
         // a bounded wait ran out (the timeout bit was set before any block
@@ -663,43 +822,41 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
         if (*(volatile uint32_t*)a.err & kErrBarrierTimeout) return;
         if (clock0) tDep += globalNs() - td0;
         // 3b. the corrected-face list and the targets of every overshooting cell
-        for (int q = gw; q < nAct; q += nw) boundCellLists(s.actList[q], m, a, s, lane, pass, passStamp, stamp);
+        for (int q0 = gw * per; q0 < nAct; q0 += nw * per) {
+            const int q = q0 + lane / gsz;
+            boundCellLists(q < nAct ? s.actList[q] : -1, gl, m, a, s, lane, pass, passStamp, stamp);
+        }
         if (!gridBarrier(s, a.err, barK)) return;
         // 4. alpha of every target cell, its updates in list order
         //    (advectionTemplates.C:164-192: own -= corr/V, nei += corr/V).
-        //    A half-warp per target, lane k on the target's k-th face; a
+        //    A group of lanes per target, lane gl on its gl-th face; a
         //    corrected face's rank is the number of corrected faces of the
-        //    cell with a smaller key, and the half-warp adds the terms up in
+        //    cell with a smaller key, and the group adds the terms up in
         //    rank order.  Targets of the bounding set join the candidates
         //    (extendMarkedCells).  Loops and shuffles run on the whole warp.
         const int nT = min(ldVol(s.ctl + kCtlTouched0 + pass), s.touchedCap);
         {
-            // a half-warp per target while every cell has at most 16 faces,
-            // else a whole warp
-            const bool wide = m.maxCellFaces > 16;
-            const int gsz = wide ? 32 : 16, per = wide ? 1 : 2;
-            const int half = wide ? 0 : (lane & 16), hl = wide ? lane : (lane & 15);
-            const unsigned hmask = wide ? 0xffffffffu : (0xffffu << half);
-            for (int r0 = (tid >> 5) * per; r0 < nT; r0 += (nth >> 5) * per) {
-                const int r = r0 + (half >> 4);
+            const unsigned hmask = gbits << base;
+            for (int r0 = gw * per; r0 < nT; r0 += nw * per) {
+                const int r = r0 + lane / gsz;
                 const bool valid = r < nT;
                 const int t = valid ? s.touched[r] : 0;
                 bool hit = false, ownSide = false, nbMixed = false;
                 unsigned key = 0xffffffffu;
-                double term = 0.0, at = 0.0, Vt = 1.0, rVt = 1.0;
+                double term = 0.0, at = 0.0;
                 if (valid) {
-                    const int k0 = m.cOff[t];
+                    const int k0 = m.uniformFaces ? t * m.uniformFaces : m.cOff[t];
+                    const int nfc = m.uniformFaces ? m.uniformFaces : m.cOff[t + 1] - k0;
                     at = a.aNew[t];
-                    Vt = m.V[t];
-                    rVt = m.rV[t];
-                    if (hl < m.cOff[t + 1] - k0) {
-                        const int g = m.cFaces[k0 + hl];
-                        const int nb = m.cSlot[k0 + hl].x;
-                        nbMixed = nb >= 0 && a.status[nb] != kStNotMixed;
+                    const double Vt = m.V[t], rVt = m.rV[t];
+                    if (gl < nfc) {
+                        const int2 sl = m.cSlot[k0 + gl];
+                        const int g = sl.y & 0x7fffffff;
+                        nbMixed = sl.x >= 0 && a.status[sl.x] != kStNotMixed;
                         if (s.faceStamp[g] == passStamp) {
                             hit = true;
                             key = s.faceKey[g];
-                            ownSide = m.own[g] == t;
+                            ownSide = sl.y >= 0;
                             term = divByRecip(s.corr[g], Vt, rVt);
                         }
                     }
@@ -708,11 +865,12 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
                 const bool need = (__ballot_sync(0xffffffffu, nbMixed) & hmask) != 0;
                 int rank = 0;
                 for (int j = 0; j < gsz; ++j) {
-                    const unsigned kj = __shfl_sync(0xffffffffu, key, half + j);
-                    if (((hits >> (half + j)) & 1u) && kj < key) ++rank;
+                    const unsigned kj = __shfl_sync(0xffffffffu, key, base + j);
+                    if (((hits >> (base + j)) & 1u) && kj < key) ++rank;
                 }
                 const bool before = overshoots(at);
-                for (int e = 0; e < m.maxCellFaces; ++e) {
+                const int nHits = __reduce_max_sync(kAll, __popc(hits));
+                for (int e = 0; e < nHits; ++e) {
                     const unsigned who = __ballot_sync(0xffffffffu, hit && rank == e) & hmask;
                     const int src = who ? __ffs(who) - 1 : lane;
                     const double x = __shfl_sync(0xffffffffu, term, src);
@@ -722,7 +880,7 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
                         else at += x;
                     }
                 }
-                if (valid && hl == 0) {
+                if (valid && gl == 0) {
                     a.aNew[t] = at;
                     aggAdd(s.ctl + kCtlOverDelta0 + pass, int(overshoots(at)) - int(before));
                     const bool inSet = need || a.status[t] != kStNotMixed;

@@ -713,18 +713,8 @@ int allocState(simplic_handle* h) {
     }
     b.info = M.alloc<int>(8);
     b.actList = M.alloc<int>(b.candCap);
-    {
-        const size_t slots = size_t(b.candCap) * h->m.maxCellFaces;
-        b.slotF = M.alloc<int>(slots);
-        b.slotFlags = M.alloc<uint8_t>(slots);
-        b.slotSucc = M.alloc<int>(slots);
-        b.slotDv = M.alloc<double>(slots);
-        b.slotPhdt = M.alloc<double>(slots);
-        b.slotMax0 = M.alloc<double>(slots);
-        b.slotThr0 = M.alloc<double>(slots);
-    }
-    b.candK = M.alloc<uint8_t>(size_t(b.candCap) * kBoundCellConstBytes);
-    b.candDepN = M.alloc<int>(b.candCap);
+    b.recBytes = int(boundRecordBytes(h->m.maxCellFaces));
+    b.rec = M.alloc<uint8_t>(size_t(b.candCap) * b.recBytes);
     b.candPending = M.alloc<int>(b.candCap);
     b.candPm = M.alloc<unsigned>(b.candCap);
     b.readyQ = M.alloc<unsigned long long>(b.candCap);
@@ -736,9 +726,7 @@ int allocState(simplic_handle* h) {
                     (void*)b.candMark, (void*)b.cellClaim, (void*)b.faceKey, (void*)b.faceStamp,
                     (void*)b.touched, (void*)b.corr, (void*)b.dvfMod, (void*)b.modStamp, (void*)b.modList,
                     (void*)b.ctl, (void*)b.barCount, (void*)b.barGen, (void*)b.info, (void*)b.actList,
-                    (void*)b.slotF, (void*)b.slotFlags, (void*)b.slotSucc, (void*)b.slotDv, (void*)b.slotPhdt,
-                    (void*)b.slotMax0, (void*)b.slotThr0, b.candK, (void*)b.candDepN, (void*)b.candPending,
-                    (void*)b.candPm, (void*)b.readyQ})
+                    (void*)b.rec, (void*)b.candPending, (void*)b.candPm, (void*)b.readyQ})
         if (!p) return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (solver state)");
     if (h->ctrl.record_cut_faces && !h->cutMask) return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (cut mask)");
     CK(h, cudaMemsetAsync(h->nMixed, 0, 2 * sizeof(int), h->stream));

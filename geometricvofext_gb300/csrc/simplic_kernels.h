@@ -64,17 +64,23 @@ enum : int {
     kCtlActive0 = 4,  // [pass] overshooting candidates
     kCtlOverDelta0 = kCtlActive0 + kMaxBoundPasses,  // [pass] change of the overshoot count
     kCtlTouched0 = kCtlOverDelta0 + kMaxBoundPasses, // [pass] target cells of the pass
-    kCtlQHead0 = kCtlTouched0 + kMaxBoundPasses,     // [pass] ready-queue entries taken
-    kCtlQTail0 = kCtlQHead0 + kMaxBoundPasses,       // [pass] ready-queue entries written
+    kCtlFree0 = kCtlTouched0 + kMaxBoundPasses,      // [pass] cells that wait for nobody
+    kCtlFreeHead0 = kCtlFree0 + kMaxBoundPasses,     // [pass] of those, taken beyond the first per warp
+    kCtlQHead0 = kCtlFreeHead0 + kMaxBoundPasses,    // [pass] released cells taken from the queue
+    kCtlQTail0 = kCtlQHead0 + kMaxBoundPasses,       // [pass] released cells written to the queue
     kCtlDone0 = kCtlQTail0 + kMaxBoundPasses,        // [pass] cells run
-    kCtlStarts0 = kCtlDone0 + kMaxBoundPasses,       // [pass] chains started from the queue
+    kCtlStarts0 = kCtlDone0 + kMaxBoundPasses,       // [pass] chains started
     kCtlSize = kCtlStarts0 + kMaxBoundPasses,
 };
-constexpr int kBoundCellConstBytes = 104;  // per-candidate constants of the cell loop
+// Record of an overshooting candidate: the constants of its loop, then one
+// slot per face; whole 128-byte lines.
+constexpr int kBoundCellConstBytes = 112;
+constexpr int kBoundSlotBytes = 48;
+constexpr size_t boundRecordBytes(int maxCellFaces) {
+    return (size_t(kBoundCellConstBytes) + size_t(kBoundSlotBytes) * maxCellFaces + 127) / 128 * 128;
+}
 
-// Scratch of the bounding kernel (per-candidate arrays have candCap rows,
-// the per-face-slot ones maxCellFaces columns: slot i * maxCellFaces + k is
-// the k-th face of candidate i in cells() order).
+// Scratch of the bounding kernel (per-candidate arrays have candCap rows).
 struct BoundBuffers {
     int* ovList;
     int* ovCount;
@@ -108,18 +114,12 @@ struct BoundBuffers {
     // phase (per face slot and per cell), the dependency counts and the
     // ready queue.
     int* actList;          // [candCap] overshooting candidates of the pass
-    int* slotF;            // [slots] face id
-    uint8_t* slotFlags;    // [slots] kSlot* bits
-    int* slotSucc;         // [slots] later overshooting candidate across a downwind face, or -1
-    double* slotDv;        // [slots] dVf at the start of the pass
-    double* slotPhdt;      // [slots] phi dt
-    double* slotMax0;      // [slots] first iteration without corrections: maxExtra
-    double* slotThr0;      // [slots] ... and the flux share
-    void* candK;           // [candCap * kBoundCellConstBytes] per-cell constants
-    int* candDepN;         // [candCap] faces on which the cell waits for an earlier cell
-    int* candPending;      // [candCap] of those, not yet published
+    uint8_t* rec;          // [candCap * recBytes] their records (BoundCellConst, BoundSlot per face)
+    int recBytes;
+    int* candPending;      // [candCap] faces on which the cell waits for an earlier cell that has not started
     unsigned* candPm;      // [candCap] faces that pass in the loop's first iteration
-    unsigned long long* readyQ;  // [candCap] (pass stamp << 32) | candidate
+    unsigned long long* readyQ;  // [candCap] (pass stamp << 32) | candidate: from the front the cells
+                                 // that wait for nobody, from the back the released ones
 };
 
 // arguments of the three plane-solve kernels

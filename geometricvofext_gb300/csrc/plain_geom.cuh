@@ -2,7 +2,6 @@
 //
 // Restates, per thread:
 //   cutFace::calcSubFace / calcSubFaceCentreAndArea   cutFace.C:37-96, 136-259
-//   cutFace::timeIntegratedFaceFlux / Area            cutFace.C:262-506
 //   cutCell::calcSubCell and helpers                  cutCell.C:37-137, 343-542
 // with the same floating-point operation order as the reference, so that a
 // translation unit built with -fmad=false reproduces the CPU results bit for
@@ -421,156 +420,23 @@ static __device__ __noinline__ void calcSubCell(const CellWS<K>& w, d3 n, double
     }
 }
 
-// |area| of a face polygon clipped by the plane (calcSubFace then
-// mag(subFaceArea)); fullMag is |face::areaNormal| of the whole face.
-__device__ __forceinline__ double clippedFaceArea(const d3* fp, int n, d3 nrm, double d, double fullMag) {
-    double dist[kMaxFacePts];
-    int nSub = 0, first = -1;
-    unsigned sub = 0;
-    for (int i = 0; i < n; ++i) {
-        dist[i] = liftedDistance(fp[i], nrm, d);
-        if (belowBits(dist[i])) {
-            ++nSub;
-            sub |= 1u << i;
-            if (first < 0) first = i;
-        }
+// What is known of a face whose points share a coordinate bit for bit: the
+// axis in bits 0-1 (3: none), bit 2 set when the rounded average of five such
+// coordinates is that coordinate, bit 3 when the whole face's area vector has
+// that component only.
+__device__ __forceinline__ uint8_t faceAxisCode(const d3* p, int n, d3 fullA) {
+    const auto comp = [](d3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); };
+    for (int k = 0; k < 3; ++k) {
+        const double x0 = comp(p[0], k);
+        bool same = true;
+        for (int i = 1; i < n; ++i) same = same && bitsOf(comp(p[i], k)) == bitsOf(x0);
+        if (!same) continue;
+        const double five = ((((x0 + x0) + x0) + x0) + x0) / 5.0;
+        bool only = true;
+        for (int q = 0; q < 3; ++q) only = only && (q == k || (bitsOf(comp(fullA, q)) << 1) == 0);
+        return uint8_t(k | (bitsOf(five) == bitsOf(x0) ? 4 : 0) | (only ? 8 : 0));
     }
-    if (nSub == n) return fullMag;
-    if (nSub == 0) return 0.0;
-    // the cut edges by position in the walk from `first`; the first two cut
-    // points on every lane at once (see clipCutFace)
-    unsigned cutE = 0;
-    for (int j = 0; j < n; ++j)
-        if (crossesBits(dist[(first + j) % n], dist[(first + j + 1) % n])) cutE |= 1u << j;
-    const auto cutPoint = [&](int j) {
-        const int cur = (first + j) % n, nxt = (first + j + 1) % n;
-        const double w = dist[cur] / (dist[cur] - dist[nxt]);
-        return fp[cur] + w * (fp[nxt] - fp[cur]);
-    };
-    const int j1 = cutE ? __ffs(cutE) - 1 : 0;
-    const unsigned rest = cutE & (cutE - 1u);
-    const int j2 = rest ? __ffs(rest) - 1 : j1;
-    const d3 c1 = cutPoint(j1), c2 = cutPoint(j2);
-    d3 sp[kMaxSubPts];
-    int ns = 0;
-    for (int j = 0; j < n; ++j) {
-        const int cur = (first + j) % n;
-        if ((sub >> cur) & 1u) sp[ns++] = fp[cur];
-        if ((cutE >> j) & 1u) sp[ns++] = (j == j1) ? c1 : (j == j2 ? c2 : cutPoint(j));
-    }
-    if (ns < 3) return fullMag;
-    return mag(fanArea(sp, ns));
-}
-
-// cutFace::timeIntegratedArea (cutFace.C:392-506)
-__device__ __forceinline__ double timeIntegratedArea(const d3* fp, int n, d3 nrm, double distance,
-                                                     const double* pTimes, double Un0, double dt, double magSf,
-                                                     double fullMag) {
-    int order[kMaxFacePts];
-    for (int i = 0; i < n; ++i) {  // stable ascending sort
-        int j = i;
-        while (j > 0 && pTimes[order[j - 1]] > pTimes[i]) {
-            order[j] = order[j - 1];
-            --j;
-        }
-        order[j] = i;
-    }
-    const double firstTime = pTimes[order[0]];
-    const double lastTime = pTimes[order[n - 1]];
-    if (lastTime <= 0.0) return magSf * dt * pos0(Un0);
-    if (firstTime >= dt) return magSf * dt * (1.0 - pos0(Un0));
-    double sortedTimes[kMaxFacePts + 2];
-    int nT = 0;
-    double tIntArea = 0.0, prevTime, subAreaOld;
-    if (firstTime > 0.0) {
-        subAreaOld = magSf * (1.0 - pos0(Un0));
-        tIntArea = subAreaOld * firstTime;
-        sortedTimes[nT++] = firstTime;
-        prevTime = firstTime;
-    } else {
-        sortedTimes[nT++] = 0.0;
-        prevTime = 0.0;
-        subAreaOld = clippedFaceArea(fp, n, nrm, distance, fullMag);
-    }
-    const double smallTime = fmax(kTSMALL / fabs(Un0), kTSMALL);
-    for (int ti = 0; ti < n; ++ti) {
-        const double timeI = pTimes[order[ti]];
-        if (timeI > (prevTime + smallTime) && timeI < dt) {
-            sortedTimes[nT++] = timeI;
-            prevTime = timeI;
-        }
-    }
-    if (lastTime > dt)
-        sortedTimes[nT++] = dt;
-    else
-        tIntArea += magSf * (dt - lastTime) * pos0(Un0);
-    for (int k = 0; k + 1 < nT; ++k) {
-        const double tauOld = sortedTimes[k];
-        const double tauNew = sortedTimes[k + 1];
-        const double deltaTau = 0.5 * (tauNew - tauOld);
-        const double subAreaNew = clippedFaceArea(fp, n, nrm, distance - tauNew * Un0, fullMag);
-        const double subAreaMid = clippedFaceArea(fp, n, nrm, distance - (tauOld + deltaTau) * Un0, fullMag);
-        tIntArea += divByRecip(deltaTau, 3.0, 1.0 / 3.0) * (subAreaOld + 4.0 * subAreaMid + subAreaNew);
-        subAreaOld = subAreaNew;
-    }
-    return tIntArea;
-}
-
-// cutFace::timeIntegratedFaceFlux (cutFace.C:262-389)
-__device__ __forceinline__ double timeIntegratedFaceFlux(const DevMesh& m, int f, d3 nrm, double distance,
-                                                         double Un0, double dt, double phi, double magSf) {
-    if (fabs(phi) <= kTSMALL) return 0.0;
-    const int q0 = m.fOff[f], n = m.fOff[f + 1] - q0;
-    d3 fp[kMaxFacePts];
-    for (int i = 0; i < n; ++i) fp[i] = ld3(m.pts, m.fPts[q0 + i]);
-    const bool flat = m.flat[f] > (1.0 - kTSMALL);
-    if (fabs(Un0 * dt) > kTSMALL) {
-        double pTimes[kMaxFacePts];
-        const double rUn0 = 1.0 / Un0;  // the arrival times share the divisor
-        for (int i = 0; i < n; ++i) {
-            const double t = divByRecip(dot(fp[i], nrm) + distance, Un0, rUn0);
-            pTimes[i] = fabs(t) < kTSMALL ? 0.0 : t;
-        }
-        if (flat) {
-            // |face::areaNormal| of the face: the per-face table holds the same bits
-            const double fullMag = mag(ld3(m.fullA, f));
-            return phi / magSf * timeIntegratedArea(fp, n, nrm, distance, pTimes, Un0, dt, magSf, fullMag);
-        }
-        d3 tri[3];
-        double tt[3];
-        tri[0] = ld3(m.Cf, f);
-        const double t0 = divByRecip(dot(tri[0], nrm) + distance, Un0, rUn0);
-        tt[0] = fabs(t0) < kTSMALL ? 0.0 : t0;
-        double dVf = 0.0;
-        for (int pi = 0; pi < n; ++pi) {
-            tri[1] = fp[pi];
-            tt[1] = pTimes[pi];
-            tri[2] = fp[(pi + 1) % n];
-            tt[2] = pTimes[(pi + 1) % n];
-            const d3 triA = 0.5 * cross(tri[1] - tri[0], tri[2] - tri[0]);
-            const double magSfTri = mag(triA);
-            const double phiTri = phi * magSfTri / magSf;
-            dVf += phiTri / magSfTri * timeIntegratedArea(tri, 3, nrm, distance, tt, Un0, dt, magSfTri, magSfTri);
-        }
-        return dVf;
-    }
-    if (flat) {
-        const double fullMag = mag(ld3(m.fullA, f));
-        const double alphaf = clippedFaceArea(fp, n, nrm, distance, fullMag) / magSf;
-        return phi * dt * alphaf;
-    }
-    d3 tri[3];
-    tri[0] = ld3(m.Cf, f);
-    double dVf = 0.0;
-    for (int pi = 0; pi < n; ++pi) {
-        tri[1] = fp[pi];
-        tri[2] = fp[(pi + 1) % n];
-        const double magSfTri = mag(0.5 * cross(tri[1] - tri[0], tri[2] - tri[0]));
-        const double phiTri = phi * magSfTri / magSf;
-        const double alphafTri = clippedFaceArea(tri, 3, nrm, distance, magSfTri) / magSfTri;
-        dVf += phiTri * dt * alphafTri;
-    }
-    return dVf;
+    return 3;
 }
 
 // The downwind faces of cell c (advection.C:131-174: phi >= 0 on an owned

@@ -16,7 +16,7 @@
 // 2,700 per warp of five hexahedra; what does not change a bit is then left
 // out (1,400 to 1,700):
 //   * on axis-aligned faces the operations whose results are known
-//     (faceAxis);
+//     (setFaceAxis);
 //   * the cuts of the bisection that a single precision estimate decides
 //     (levelEstimate): the two ends of the bracket are the only levels cut;
 //   * the sub-faces in the final cut, whose volume nobody reads;
@@ -71,7 +71,7 @@ struct GroupCell {
     using Indices = typename FaceIndices<(K::kFacePts > 4)>::type;
     Indices fidx;
     d3 fullC, fullA;       // face::centre / areaNormal of the whole face
-    int axis;              // the axis the face is constant on (-1: none), see faceAxis
+    int axis;              // the axis the face is constant on (-1: none), see setFaceAxis
     bool five, fullFlat;   // a pentagon's average keeps the constant; fullA has that component only
     double x0, x3;         // the constant coordinate, (x0 + x0) + x0
     __device__ __forceinline__ unsigned groupBits(unsigned ballot) const {
@@ -159,27 +159,17 @@ __device__ __forceinline__ double absAtLeastVSmall(double x) {
 //     nothing but the sign of a zero, which no result shows.
 // A fan triangle then takes 18 operations instead of about 45.  u, v are the
 // two axes after the constant one in cyclic order.
+// code: faceAxisCode of the lane's face.
 template <class K, int G>
-__device__ __forceinline__ void faceAxis(GroupCell<K, G>& w) {
-    w.axis = -1;
-    w.five = w.fullFlat = false;
+__device__ __forceinline__ void setFaceAxis(GroupCell<K, G>& w, unsigned code) {
+    w.axis = (code & 3) == 3 ? -1 : int(code & 3);
+    w.five = code & 4;
+    w.fullFlat = code & 8;
     w.x0 = w.x3 = 0.0;
-    if (w.fsz == 0) return;
-    const double* p0 = w.sh->P[w.g][w.vertex(0)];
-    unsigned same = 7u;
-    for (int i = 1; i < w.fsz; ++i) {
-        const double* p = w.sh->P[w.g][w.vertex(i)];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (bitsOf(p[k]) != bitsOf(p0[k])) same &= ~(1u << k);
+    if (w.axis >= 0) {
+        w.x0 = w.sh->P[w.g][w.vertex(0)][w.axis];
+        w.x3 = (w.x0 + w.x0) + w.x0;
     }
-    if (!same) return;
-    w.axis = __ffs(same) - 1;
-    w.x0 = p0[w.axis];
-    w.x3 = (w.x0 + w.x0) + w.x0;
-    w.five = bitsOf(divCount1((w.x3 + w.x0) + w.x0, 5)) == bitsOf(w.x0);
-    const long long ax = bitsOf(w.fullA.x) << 1, ay = bitsOf(w.fullA.y) << 1, az = bitsOf(w.fullA.z) << 1;
-    w.fullFlat = (w.axis == 0 || ax == 0) && (w.axis == 1 || ay == 0) && (w.axis == 2 || az == 0);
 }
 
 // The cell's points, and the lane's face in cells() order as local point
@@ -214,6 +204,7 @@ __device__ __forceinline__ bool groupLoad(const DevMesh& m, int c, bool act, Gro
         }
     }
     __syncwarp();
+    unsigned code = 3;  // (no face)
     if (w.l < w.nf) {
         const int f = m.cFaces[f0 + w.l];
         const int q0 = m.fOff[f], n = m.fOff[f + 1] - q0;
@@ -233,12 +224,16 @@ __device__ __forceinline__ bool groupLoad(const DevMesh& m, int c, bool act, Gro
             }
             w.fullC = ld3(m.fullC, f);
             w.fullA = ld3(m.fullA, f);
+            code = m.faceAxis[f];
         }
     }
     // all lanes of the group agree
     const bool good = w.groupBits(__ballot_sync(kAllLanes, !ok)) == 0;
-    if (!good) w.np = w.nf = w.fsz = 0;
-    faceAxis(w);
+    if (!good) {
+        w.np = w.nf = w.fsz = 0;
+        code = 3;
+    }
+    setFaceAxis(w, code);
     return good;
 }
 
@@ -319,7 +314,7 @@ __device__ __forceinline__ bool groupLoadSplit(const DevMesh& m, int c, bool act
 template <class K, int G>
 __device__ __forceinline__ void groupSplitFace(const DevMesh& m, int c, GroupCell<K, G>& w) {
     GroupShared<K, G>& s = *w.sh;
-    faceAxis(w);  // (no face yet: none)
+    setFaceAxis(w, 3);  // (no face yet)
     if (!(w.l < w.nf)) return;
     const int code = s.faceOf[w.g][w.l];
     const int k = code & 0xff, t = (code >> 8) - 1;
@@ -359,7 +354,7 @@ __device__ __forceinline__ void groupSplitFace(const DevMesh& m, int c, GroupCel
     }
     w.fullC = faceCentreOF(fp, w.fsz);
     w.fullA = faceAreaNormalOF(fp, w.fsz);
-    faceAxis(w);
+    setFaceAxis(w, faceAxisCode(fp, w.fsz, w.fullA));
 }
 
 // calcSubFaceCentreAndArea (fanCentreArea of the serial form) of the polygon
@@ -400,7 +395,7 @@ __device__ __forceinline__ void groupFan(const GroupShared<K, G>& s, int lane, i
     }
 }
 
-// The same on an axis-aligned face (faceAxis): centre as (constant axis, u,
+// The same on an axis-aligned face (setFaceAxis): centre as (constant axis, u,
 // v) in cen and the area's one component.  False where a condition of the
 // shortcut does not hold (more than five points, areas too small or of both
 // signs); the general fan decides then.

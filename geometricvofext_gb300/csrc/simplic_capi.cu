@@ -579,10 +579,15 @@ int uploadMesh(simplic_handle* h, const simplic_mesh_desc* d, const HostMesh& hm
     double* flat = h->mem.alloc<double>(nf);
     double* fullC = h->mem.alloc<double>(size_t(3) * nf);
     double* fullA = h->mem.alloc<double>(size_t(3) * nf);
-    if (!flat || !fullC || !fullA) return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (face data)");
+    uint8_t* faceAxis = h->mem.alloc<uint8_t>(nf);
+    int* warped = h->mem.alloc<int>(1);
+    if (!flat || !fullC || !fullA || !faceAxis || !warped)
+        return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (face data)");
     m.flat = flat;
     m.fullC = fullC;
     m.fullA = fullA;
+    m.faceAxis = faceAxis;
+    CK(h, cudaMemsetAsync(warped, 0, sizeof(int), h->stream));
     {
         double* rV = h->mem.alloc<double>(nc);
         if (!rV) return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (reciprocal volumes)");
@@ -590,8 +595,10 @@ int uploadMesh(simplic_handle* h, const simplic_mesh_desc* d, const HostMesh& hm
         launchRecipVolume(m, rV, h->stream);
     }
     timedLaunch(h, kKFlat, [&] { launchFaceFlatness(m, h->Sf, flat, h->stream); });
-    timedLaunch(h, kKFaceFull, [&] { launchFaceFull(m, fullC, fullA, h->stream); });
+    timedLaunch(h, kKFaceFull, [&] { launchFaceFull(m, fullC, fullA, faceAxis, warped, h->stream); });
     CK(h, cudaGetLastError());
+    CK(h, cudaMemcpyAsync(&m.warped, warped, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaStreamSynchronize(h->stream));
     m.splitClass = nullptr;
     m.splitClassMask = 0;
     if (h->ctrl.split_warped_face) {

@@ -307,6 +307,8 @@ struct DevMesh {
     const double* pbW;
     const double* fullC;     // [3 nf] face::centre of each face (for fully submerged faces)
     const double* fullA;     // [3 nf] face::areaNormal of each face
+    const uint8_t* faceAxis; // [nf] what is known of an axis-aligned face (faceAxisCode)
+    int32_t warped;          // the mesh has a warped face (flatness <= 1 - TSMALL)
     const uint8_t* cellClass;  // [nc] 0 CapsHex, 1 CapsPoly, 2 CapsBig
     int32_t classMask;         // bit k: the mesh has cells of class k
     const uint8_t* splitClass; // [nc] class of the splitWarpedFace workspace (when enabled)

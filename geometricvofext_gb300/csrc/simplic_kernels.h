@@ -180,7 +180,8 @@ void launchUpdate(const StepArgs& a, cudaStream_t st);
 cudaError_t launchBound(const StepArgs& a, const BoundBuffers& b, cudaStream_t st);
 void launchBruteForce(const StepArgs& a, cudaStream_t st);
 void launchFaceFlatness(const DevMesh& m, const double* Sf, double* flat, cudaStream_t st);
-void launchFaceFull(const DevMesh& m, double* fullC, double* fullA, cudaStream_t st);
+// also the axis codes, and in *warped whether a face is warped (flat is ready)
+void launchFaceFull(const DevMesh& m, double* fullC, double* fullA, uint8_t* faceAxis, int* warped, cudaStream_t st);
 void launchRecipVolume(const DevMesh& m, double* rV, cudaStream_t st);
 // LS stencil rows of all cells: lengths (count) or the rows at off
 void launchStencilRows(const DevMesh& m, bool count, int* len, const int* off, int* rows, cudaStream_t st);

@@ -39,6 +39,7 @@ UNITS = {
     "mixed_kernels.cu": [],
     # tensor-core layers of the learned-normal network, its inputs and samples
     "mlp_kernels.cu": [],
+    "mlp_train.cu": [],
     "learned_kernels.cu": [],
 }
 

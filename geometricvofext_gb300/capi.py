@@ -79,7 +79,7 @@ EXPORTS = (
     "simplic_set_kernel_timing", "simplic_kernel_times", "simplic_reset_kernel_times",
     "simplic_bound_info", "simplic_bound_profile", "simplic_mesh_info", "simplic_rdf_iterations", "simplic_get_interface_polygons",
     "simplic_map_alpha_field", "simplic_mixed_cells_noalloc", "simplic_mlp_gemm", "simplic_mlp_forward",
-    "simplic_mlp_samples",
+    "simplic_mlp_samples", "simplic_mlp_train_forward", "simplic_mlp_train_backward", "simplic_mlp_loss",
     "simplic_set_network", "simplic_network_stats", "simplic_network_info", "simplic_network_inputs",
 )
 N_KERNELS = 14
@@ -136,6 +136,9 @@ def load(build_if_needed: bool = True):
     L.simplic_mlp_gemm.argtypes = [vp, i32, vp, i32, i32, i32, i32, i32, vp, i32, vp, vp, i32, vp, i32, vp, i32,
                                    i32, vp, vp]
     L.simplic_mlp_forward.argtypes = [vp, vp, i32, vp, vp, vp, i32, vp, vp]
+    L.simplic_mlp_train_forward.argtypes = [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp]
+    L.simplic_mlp_train_backward.argtypes = [vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, i32, vp, vp]
+    L.simplic_mlp_loss.argtypes = [vp, vp, vp, i32, C.c_float, vp, vp, vp]
     L.simplic_mlp_samples.argtypes = [h, C.c_uint64, i32, i32, vp, vp]
     L.simplic_set_network.argtypes = [h, vp, vp, C.c_float]
     L.simplic_network_stats.argtypes = [h, _ip]

@@ -26,80 +26,10 @@
 #include <cstdint>
 
 #include "../../include/simplic_mlp.h"
+#include "mlp_tc.cuh"
 
 namespace simplic {
 namespace {
-
-constexpr int kTileM = 128;
-constexpr int kTileK = 64;
-constexpr int kThreads = 128;
-constexpr long long kWaitLimit = 1ll << 22;  // try_wait polls (a few seconds at most)
-
-__device__ __forceinline__ uint32_t smemAddr(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// Byte offset of element (r, k) of a K-major tile with kTileK columns in the
-// no-swizzle canonical layout.
-__device__ __forceinline__ uint32_t coreOffset(int r, int k) {
-    return uint32_t((r >> 3) * 1024 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
-}
-
-// tcgen05 shared-memory matrix descriptor: start address, leading (K) and
-// stride (row) byte offsets, version bits 46-48 = 0b001, no swizzle.
-__device__ __forceinline__ uint64_t smemDesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= uint64_t((addr >> 4) & 0x3FFF);
-    d |= uint64_t((lbo >> 4) & 0x3FFF) << 16;
-    d |= uint64_t((sbo >> 4) & 0x3FFF) << 32;
-    d |= uint64_t(1) << 46;
-    return d;
-}
-
-// Instruction descriptor of kind::f16: D = F32, A = B = BF16, both K-major,
-// M = 128, N = n.
-__host__ __device__ constexpr uint32_t instrDesc(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(kTileM >> 4) << 24);
-}
-
-__device__ __forceinline__ void mbarInit(uint64_t* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
-}
-
-// Bounded wait for the completion of the phase with the given parity.
-__device__ __forceinline__ bool mbarWait(uint64_t* bar, uint32_t parity) {
-    const uint32_t a = smemAddr(bar);
-    for (long long i = 0; i < kWaitLimit; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
-// tanh form of GELU with the hardware tanh (tanh.approx.f32, relative error
-// about 2^-11, far below the BF16 rounding of the activations); training
-// and inference use the same function
-__device__ __forceinline__ float tanhHw(float x) {
-    float y;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float geluF(float z) {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    return 0.5f * z * (1.f + tanhHw(k0 * (z + k1 * z * z * z)));
-}
-__device__ __forceinline__ float geluGradF(float z) {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    const float u = k0 * (z + k1 * z * z * z);
-    const float t = tanhHw(u);
-    const float du = k0 * (1.f + 3.f * k1 * z * z);
-    return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * du;
-}
 
 struct GemmArgs {
     const __nv_bfloat16* A;
@@ -285,14 +215,6 @@ __global__ void __launch_bounds__(kThreads) kGemmTN(GemmArgs g) {
 // (bias, GELU, BF16) writes the next layer's input back into the same tile.
 // Persistent over 128-row tiles; the row count is read on the device.
 // ---------------------------------------------------------------------------
-constexpr int kNetWidth = 128;
-constexpr int kNetOut = 16;  // rows of the output layer evaluated (4 used)
-constexpr uint32_t kNetSbo = (kNetWidth / 8) * 128;  // row-adjacent core matrices for K = 128
-
-__device__ __forceinline__ uint32_t coreOffset128(int r, int k) {
-    return uint32_t((r >> 3) * kNetSbo + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
-}
-
 // rows x 128 BF16 from global memory into the core-matrix layout, 16 bytes
 // per asynchronous copy, all in flight at once; rows from validRows on are
 // zero-filled (nothing is read for them).

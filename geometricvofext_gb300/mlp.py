@@ -8,9 +8,9 @@ GELU between layers; outputs 0-2 correct the least-squares normal (the
 normal is normalise(n_ls + y[0:3])), output 3 is the plane constant
 (d + n.C) / h, outputs 4-127 are unused (their weights stay zero).
 
-Every matrix product of training and inference runs in ``simplic_mlp_gemm``
-(tcgen05.mma, csrc/mlp_kernels.cu); torch provides device memory and the
-elementwise glue (the loss gradient of the four outputs and Adam).  Training
+Every matrix product of training and inference runs in the tcgen05 kernels
+(csrc/mlp_train.cu, csrc/mlp_kernels.cu); torch provides device memory and
+Adam.  Training
 samples come from ``Simplic.samples`` (the step's own cut-cell volumes).
 The product path fails if the CUDA library is missing.
 
@@ -88,6 +88,16 @@ def loss_and_grad(Y, T, X):
     constant) and its gradient dL/dY (FP32, zero beyond the outputs)."""
     import torch
 
+    if _kernel_rows(Y, torch.float32, WIDTH) and _kernel_rows(T, torch.float32, N_OUT) and \
+            _kernel_rows(X, torch.bfloat16, WIDTH) and Y.shape[0] == T.shape[0] == X.shape[0] > 0:
+        dY = torch.empty_like(Y)
+        loss = torch.empty(1, dtype=torch.float64, device=Y.device)
+        st = torch.cuda.current_stream(Y.device).cuda_stream
+        r = capi.load().simplic_mlp_loss(Y.data_ptr(), X.data_ptr(), T.data_ptr(), Y.shape[0], D_WEIGHT,
+                                         dY.data_ptr(), loss.data_ptr(), st)
+        if r != 0:
+            raise RuntimeError(f"simplic_mlp_loss failed ({r})")
+        return loss.item(), dY
     y = Y[:, :N_OUT].detach().requires_grad_(True)
     nn = normals_from_outputs(X, y)
     cos = (nn * T[:, :3]).sum(1)
@@ -96,6 +106,12 @@ def loss_and_grad(Y, T, X):
     dY = torch.zeros_like(Y)
     dY[:, :N_OUT] = g
     return float(L.item()), dY
+
+
+def _kernel_rows(t, dtype, width):
+    """Rows the training kernels can read: CUDA, contiguous, 16-byte aligned."""
+    return t.is_cuda and t.dtype == dtype and t.dim() == 2 and t.shape[1] == width and t.is_contiguous() \
+        and t.data_ptr() % 16 == 0
 
 
 class Trainer:
@@ -119,14 +135,13 @@ class Trainer:
         self.err = torch.zeros(1, dtype=torch.int32, device=self.dev)
         f32, bf = torch.float32, torch.bfloat16
         B = batch
-        self.Z = [torch.empty((B, WIDTH), dtype=f32, device=self.dev) for _ in range(N_LAYERS - 1)]
-        self.H = [torch.empty((B, WIDTH), dtype=bf, device=self.dev) for _ in range(N_LAYERS - 1)]
-        self.HT = [torch.empty((WIDTH, B), dtype=bf, device=self.dev) for _ in range(N_LAYERS - 1)]
+        L = N_LAYERS - 1
+        # pre-activations, transposed activations and, for the backward pass,
+        # the transposed input and dZ of every layer
+        self.Z = torch.empty((L, B, WIDTH), dtype=f32, device=self.dev)
+        self.HT = torch.empty((L, WIDTH, B), dtype=bf, device=self.dev)
         self.Y = torch.empty((B, WIDTH), dtype=f32, device=self.dev)
-        self.dZ = torch.empty((B, WIDTH), dtype=bf, device=self.dev)
-        self.dZT = torch.empty((WIDTH, B), dtype=bf, device=self.dev)
-        self.dZ2 = torch.empty((B, WIDTH), dtype=bf, device=self.dev)
-        self.dZ2T = torch.empty((WIDTH, B), dtype=bf, device=self.dev)
+        self.scratch = torch.empty((N_LAYERS + 1, WIDTH, B), dtype=bf, device=self.dev)
         self.gW = torch.zeros_like(self.W)
         self.gb = torch.zeros_like(self.b)
         self._refresh()
@@ -135,35 +150,36 @@ class Trainer:
         self.Wb = self.W.to(self.t.bfloat16).contiguous()
         self.WbT = self.W.transpose(1, 2).to(self.t.bfloat16).contiguous()
 
+    def _rows(self, t, dtype):
+        """t as rows the kernels can read, at most the trainer's batch."""
+        t = t.to(dtype).contiguous()
+        if t.data_ptr() % 16:
+            t = t.clone()
+        if not t.is_cuda or t.dim() != 2 or t.shape[1] != WIDTH or t.shape[0] > self.B:
+            raise RuntimeError(f"rows of shape {tuple(t.shape)} on {t.device}: [at most {self.B}, {WIDTH}] on the GPU")
+        return t
+
     def forward(self, X):
-        """X BF16 [B, 128] -> Y FP32 [B, 128] (keeps Z, H for backward)."""
-        A = X
-        for l in range(N_LAYERS - 1):
-            gemm(A, self.Wb[l], BIAS_GELU, D=self.Z[l], bias=self.b[l], H=self.H[l], HT=self.HT[l], err=self.err)
-            A = self.H[l]
-        gemm(A, self.Wb[-1], BIAS, D=self.Y, bias=self.b[-1], err=self.err)
+        """X BF16 [B, 128] -> Y FP32 [B, 128] (keeps Z, HT for backward)."""
+        X = self._rows(X, self.t.bfloat16)
+        st = self.t.cuda.current_stream(self.dev).cuda_stream
+        r = capi.load().simplic_mlp_train_forward(
+            X.data_ptr(), X.shape[0], self.B, self.Wb.data_ptr(), self.b.data_ptr(), self.Z.data_ptr(),
+            self.HT.data_ptr(), self.Y.data_ptr(), self.err.data_ptr(), st)
+        if r != 0:
+            raise RuntimeError(f"simplic_mlp_train_forward failed ({r})")
         return self.Y
 
     def backward(self, X, dY, split_k=8):
         """Gradients of all weights and biases for dL/dY (FP32 [B, 128])."""
-        t = self.t
-        XT = X.transpose(0, 1).contiguous()
-        self.gW.zero_()
-        dYb = dY.to(t.bfloat16)
-        dYT = dYb.transpose(0, 1).contiguous()
-        L = N_LAYERS - 1
-        # output layer
-        gemm(dYT, self.HT[L - 1], ATOMIC, D=self.gW[L], split_k=split_k, err=self.err)
-        self.gb[L] = dY.sum(0)
-        gemm(dYb, self.WbT[L], GELU_BACKWARD, H=self.dZ, HT=self.dZT, Zin=self.Z[L - 1], err=self.err)
-        cur, curT, nxt, nxtT = self.dZ, self.dZT, self.dZ2, self.dZ2T
-        for l in range(L - 1, -1, -1):
-            inT = self.HT[l - 1] if l > 0 else XT
-            gemm(curT, inT, ATOMIC, D=self.gW[l], split_k=split_k, err=self.err)
-            self.gb[l] = cur.float().sum(0)
-            if l > 0:
-                gemm(cur, self.WbT[l], GELU_BACKWARD, H=nxt, HT=nxtT, Zin=self.Z[l - 1], err=self.err)
-                cur, curT, nxt, nxtT = nxt, nxtT, cur, curT
+        X, dY = self._rows(X, self.t.bfloat16), self._rows(dY, self.t.float32)
+        st = self.t.cuda.current_stream(self.dev).cuda_stream
+        r = capi.load().simplic_mlp_train_backward(
+            X.data_ptr(), dY.data_ptr(), X.shape[0], self.B, self.WbT.data_ptr(), self.Z.data_ptr(),
+            self.HT.data_ptr(), self.scratch.data_ptr(), self.gW.data_ptr(), self.gb.data_ptr(), split_k,
+            self.err.data_ptr(), st)
+        if r != 0:
+            raise RuntimeError(f"simplic_mlp_train_backward failed ({r})")
         return self.gW, self.gb
 
     def adam(self, lr=None, b1=0.9, b2=0.999, eps=1e-8):

@@ -45,6 +45,27 @@ int simplic_mlp_gemm(const void* A, int32_t lda, const void* B, int32_t ldb, int
 int simplic_mlp_forward(const void* X, const int32_t* M, int32_t maxRows, const void* W, const float* b, float* Y,
                         int32_t ldy, uint32_t* err, void* stream);
 
+/* Training: one gradient evaluation of the network on M rows.  W and WT are
+ * BF16 [4][128][128] (row = output unit, and transposed), b FP32 [4][128].
+ * ld >= M is the row capacity of the buffers: Z FP32 [3][ld][128] and HT BF16
+ * [3][128][ld] (pre-activations and transposed activations of the hidden
+ * layers), Y and dY FP32 [ld][128], scratch BF16 [5][128][ld].  X is
+ * contiguous.  All bases 16-byte aligned.  The backward pass needs M a
+ * multiple of 64 and ld of 8; gW FP32 [4][128][128] and gb FP32 [4][128] are
+ * overwritten; splitK is the least number of parts the rows are split into
+ * for the weight gradients. */
+int simplic_mlp_train_forward(const void* X, int32_t M, int32_t ld, const void* W, const float* b, float* Z, void* HT,
+                              float* Y, uint32_t* err, void* stream);
+int simplic_mlp_train_backward(const void* X, const float* dY, int32_t M, int32_t ld, const void* WT, const float* Z,
+                               const void* HT, void* scratch, float* gW, float* gb, int32_t splitK, uint32_t* err,
+                               void* stream);
+/* Loss of the outputs Y (FP32 [n][128]) against T (FP32 [n][4]: normal, plane
+ * constant) on the inputs X, into *loss (device), and its gradient dY: mean of
+ * 1 - cos of the angle between normalise(n_ls + y[0:3]) and T[0:3], plus
+ * dWeight times the mean square of y[3] - T[3]. */
+int simplic_mlp_loss(const float* Y, const void* X, const float* T, int32_t n, float dWeight, float* dY, double* loss,
+                     void* stream);
+
 /* Training samples on the handle's mesh (enqueued on the handle's stream):
  * count rows of network input X (BF16 [count][128]) and targets T (FP32
  * [count][4]: unit normal, (d + n.C) / h).  Each sample is a random plane

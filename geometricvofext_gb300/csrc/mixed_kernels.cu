@@ -8,7 +8,8 @@
 //     plane constant of its cuboid (the cut volume inverted region by region,
 //     checked against alpha); any other cell takes the reference's own steps
 //     (cutCell.C:611-799: the bracket of two vertex levels, the cubic through
-//     the 1/3 and 2/3 cuts, Newton on the cubic), the plain form's kernel;
+//     the 1/3 and 2/3 cuts, Newton on the cubic): the plain form's kernel, or
+//     on meshes with warped faces this file's;
 //   * Simpson fluxes: the clipped face areas of cutFace::timeIntegratedArea
 //     (cutFace.C:392-506) in FP32 on face-local coordinates (points shifted
 //     by the face centre, plane constant shifted with them), fan sums with
@@ -374,6 +375,132 @@ __global__ void __launch_bounds__(128) kBoxPlanes(DevMesh m, PlaneArgs p, int* _
     }
 }
 
+// Vertex distances -n.x of the cell points and their stable descending
+// order (cutCell.C:644-670).
+template <class K>
+__device__ __forceinline__ void vertexOrder(const CellWS<K>& w, d3 nI, double* vd, int* order) {
+    const int np = w.np;
+    for (int i = 0; i < np; ++i) vd[i] = -dot(nI, w.P[i]);
+    for (int i = 0; i < np; ++i) {
+        int j = i;
+        while (j > 0 && vd[order[j - 1]] < vd[i]) {
+            order[j] = order[j - 1];
+            --j;
+        }
+        order[j] = i;
+    }
+}
+
+// cutCell::findSignedDistance (cutCell.C:611-799), splitWarpedFace = false.
+// d/ic/is are written exactly where the reference writes interfaceD/C/S.
+template <class K>
+__device__ __forceinline__ int findSignedDistance(const CellWS<K>& w, double alphaI, d3 nI, double& dOut, d3& icOut,
+                                                  d3& isOut, uint32_t& err) {
+    if (mag(nI) < kTSMALL) return int(sgn(0.5 - alphaI));
+    const int np = w.np;
+    double vd[K::kPts];
+    int order[K::kPts];
+    vertexOrder(w, nI, vd, order);
+    Bracket br;
+    br.lowD = vd[order[0]];
+    br.upD = vd[order[np - 1]];
+    br.lowA = 0.0;
+    br.upA = 1.0;
+    int lowLabel = 0, upLabel = np - 1;
+    SubCell sc;
+    while ((upLabel - lowLabel) > 1) {
+        const int midLabel = (upLabel + lowLabel + 1) >> 1;
+        const double midDistance = vd[order[midLabel]];
+        calcSubCell(w, nI, midDistance, sc, err);
+        const double midAlpha = sc.vof;
+        if (fabs(midAlpha - alphaI) < kTSMALL) {
+            dOut = midDistance;
+            icOut = sc.ic;
+            isOut = sc.is;
+            return sc.status;
+        }
+        if (midAlpha > alphaI) {
+            upLabel = midLabel;
+            br.upD = midDistance;
+            br.upA = midAlpha;
+        } else {
+            lowLabel = midLabel;
+            br.lowD = midDistance;
+            br.lowA = midAlpha;
+        }
+    }
+    if (fabs(br.lowD - br.upD) < kTSMALL) {
+        const double midDistance = 0.5 * (br.lowD + br.upD);
+        calcSubCell(w, nI, midDistance, sc, err);
+        dOut = midDistance;
+        icOut = sc.ic;
+        isOut = sc.is;
+        return sc.status;
+    }
+    const double deltaDistance = (br.upD - br.lowD) / 3.0;
+    calcSubCell(w, nI, br.lowD + deltaDistance, sc, err);
+    const double v13 = sc.vof;
+    calcSubCell(w, nI, br.lowD + 2.0 * deltaDistance, sc, err);
+    const double v23 = sc.vof;
+    const double distance0 = cubicDistance(br, v13, v23, alphaI);
+    calcSubCell(w, nI, distance0, sc, err);
+    dOut = distance0;
+    icOut = sc.ic;
+    isOut = sc.is;
+    return sc.status;
+}
+
+// Meshes with warped faces: one thread per cell.  The sub-cells of a warped
+// cell do not close exactly, the cubic through the cuts may have no root in
+// its bracket, and Newton on it then ends (after its hundred trips) wherever
+// round-off sends it: on such a cell the plane changes by a per cent of the
+// cell with any change of the operation order, so these meshes do not take
+// the general solve's (on rough fields some ten cells in 27,000 would).
+// Meshes with flat faces agree to 1e-10 either way.  One instantiation per
+// cell class (workspace caps K); a launch handles the mixed cells of its class.
+template <class K>
+__global__ void __launch_bounds__(128) kPlaneSolveMixed(DevMesh m, PlaneArgs p, int cls) {
+    const int nm = *p.nMixed;
+    uint32_t err = 0;
+    for (int i = spreadFirst(); i < nm; i += spreadStride()) {
+        const int c = p.mixed[i];
+        if (m.classMask != (1 << cls) && m.cellClass[c] != cls) continue;
+        CellWS<K> w;
+        double d = 0.0;
+        d3 ic = mk(0, 0, 0), is = mk(0, 0, 0);
+        int st;
+        const double alphaI = p.alpha[c];
+        const d3 nI = ld3(p.nrm, i);
+        const unsigned bx = m.boxCorner[c];
+        if (bx && alphaI > 0.0 && alphaI < 1.0) {
+            const int p0 = m.cpOff[c];
+            const d3 lo = ld3(m.pts, m.cPts[p0 + ((bx >> 3) & 7)]), hi = ld3(m.pts, m.cPts[p0 + (bx & 7)]);
+            if (boxPlane(nI, lo, hi, alphaI, m.V[c], d, ic, is)) {
+                p.mStatus[i] = 0;
+                p.status[c] = 0;
+                p.dOut[i] = d;
+                st3(p.icOut, i, ic);
+                st3(p.isOut, i, is);
+                continue;
+            }
+        }
+        if (!loadCell(m, c, w)) {
+            err |= kErrSubFaceOverflow;
+            st = 1;
+        } else if (mag(nI) < kTSMALL) {
+            st = int(sgn(0.5 - alphaI));
+        } else {
+            st = findSignedDistance(w, alphaI, nI, d, ic, is, err);
+        }
+        p.mStatus[i] = int8_t(st);
+        p.status[c] = int8_t(st);
+        p.dOut[i] = d;
+        st3(p.icOut, i, ic);
+        st3(p.isOut, i, is);
+    }
+    if (err) atomicOr(p.err, err);
+}
+
 // ---------------------------------------------------------------------------
 // Simpson fluxes: FP32 clipping on face-local coordinates
 // ---------------------------------------------------------------------------
@@ -704,11 +831,24 @@ __global__ void __launch_bounds__(128) kInterfaceUn0Mixed(DevMesh m, const int* 
 
 }  // namespace
 
+static void planeSolveMixedAll(const DevMesh& m, const PlaneArgs& p, cudaStream_t st) {
+    if (m.classMask & 1)
+        kPlaneSolveMixed<CapsHex><<<residentGridM(kPlaneSolveMixed<CapsHex>, 128), 128, 0, st>>>(m, p, 0);
+    if (m.classMask & 2)
+        kPlaneSolveMixed<CapsPoly><<<residentGridM(kPlaneSolveMixed<CapsPoly>, 128), 128, 0, st>>>(m, p, 1);
+    if (m.classMask & 4)
+        kPlaneSolveMixed<CapsBig><<<residentGridM(kPlaneSolveMixed<CapsBig>, 128), 128, 0, st>>>(m, p, 2);
+}
+
 void launchLsNormalMixed(const StepArgs& a, cudaStream_t st) {
     kLsNormalMixed<<<residentGridM(kLsNormalMixed, 128), 128, 0, st>>>(a.m, a.aCur, a.mixed, a.nMixed, a.nrm, a.err);
 }
 
 void launchPlaneSolveMixed(const StepArgs& a, bool boxes, cudaStream_t st) {
+    if (a.m.warped) {
+        planeSolveMixedAll(a.m, planeArgs(a), st);
+        return;
+    }
     if (!boxes) {  // no box cell in the mesh
         launchPlaneSolve(a, st);
         return;

@@ -809,14 +809,13 @@ __device__ __forceinline__ void levelEstimate(d3 n, float Lx, float Ly, float Lz
     dn = flip ? more : less;
 }
 
-// cutCell::findSignedDistance (cutCell.C:611-799): the bracket of two vertex
-// levels by bisection, the cuts at 1/3 and 2/3, Newton on the cubic, the
-// final cut.  d / ic / is are set where the reference writes interfaceD/C/S.
+// The vertex levels of the group's cell in descending order (sv), and which
+// of them cut clearly more (above) or less (under) than alpha.  False for an
+// idle group and for a cell without a normal (status in st).
 template <class K, int G>
-__device__ __forceinline__ int groupSignedDistance(GroupCell<K, G>& w, bool act, unsigned box, double alphaI, d3 nI,
-                                                   double& dOut, d3& icOut, d3& isOut, uint32_t& err) {
+__device__ __forceinline__ bool groupLevels(GroupCell<K, G>& w, bool act, unsigned box, double alphaI, d3 nI, int& st,
+                                            unsigned& above, unsigned& under) {
     GroupShared<K, G>& s = *w.sh;
-    int st = 0;
     // mag(nI) < TSMALL, without the root where one component alone decides
     if (act && absBelow(nI.x, 2.0 * kTSMALL) && absBelow(nI.y, 2.0 * kTSMALL) && absBelow(nI.z, 2.0 * kTSMALL) &&
         mag(nI) < kTSMALL) {
@@ -847,16 +846,11 @@ __device__ __forceinline__ int groupSignedDistance(GroupCell<K, G>& w, bool act,
         s.sv[w.g][rank] = -s.pd[w.g][i];
     }
     __syncwarp();
-    const double* sv = s.sv[w.g];
-    Bracket br;
-    br.lowA = 0.0;
-    br.upA = 1.0;
-    int lowLabel = 0, upLabel = np - 1;
-    bool lowKnown = true, upKnown = true;  // lowA / upA are the cut volumes of the levels
     // Box cells: which levels cut clearly more or less than alpha, from the
     // volume fraction of the box below each level in single precision
     // (lane l on level l + 1).
-    unsigned above = 0, under = 0;
+    above = under = 0;
+    const double* sv = s.sv[w.g];
     if (K::kFaces == 6) {
         bool up = false, dn = false;
         if (act && box && l < 6) {
@@ -872,6 +866,26 @@ __device__ __forceinline__ int groupSignedDistance(GroupCell<K, G>& w, bool act,
         above = w.groupBits(__ballot_sync(kAllLanes, up)) << 1;
         under = w.groupBits(__ballot_sync(kAllLanes, dn)) << 1;
     }
+    return act;
+}
+
+// cutCell::findSignedDistance (cutCell.C:611-799): the bracket of two vertex
+// levels by bisection, the cuts at 1/3 and 2/3, Newton on the cubic, the
+// final cut.  d / ic / is are set where the reference writes interfaceD/C/S.
+template <class K, int G>
+__device__ __forceinline__ int groupSignedDistance(GroupCell<K, G>& w, bool act, unsigned box, double alphaI, d3 nI,
+                                                   double& dOut, d3& icOut, d3& isOut, uint32_t& err) {
+    GroupShared<K, G>& s = *w.sh;
+    int st = 0;
+    unsigned above, under;
+    act = groupLevels(w, act, box, alphaI, nI, st, above, under);
+    const int np = act ? w.np : 0;
+    const double* sv = s.sv[w.g];
+    Bracket br;
+    br.lowA = 0.0;
+    br.upA = 1.0;
+    int lowLabel = 0, upLabel = np - 1;
+    bool lowKnown = true, upKnown = true;  // lowA / upA are the cut volumes of the levels
     // the bisection as far as the clear levels decide it
     const auto settle = [&] {
         while (upLabel - lowLabel > 1) {
@@ -979,6 +993,147 @@ __device__ __forceinline__ int groupSignedDistance(GroupCell<K, G>& w, bool act,
         }
     }
     return st;
+}
+
+// The same for one cell on all groups of the warp, every group with the cell
+// loaded: cuts that do not wait for one another run at once, a group each.
+// A bisection cuts its next level and those that may follow it (group g the
+// g-th node, breadth first, of the tree of levels below the bracket) and then
+// takes the serial decisions as far as the volumes are there; the unknown ends
+// of the bracket and its thirds go together.  The planes are the same: a
+// level's volume does not depend on when it is cut, and one that is never
+// asked for is not looked at.  For lists that leave warps idle: a box cell
+// waits for two cuts in a row instead of five, any hexahedron for four instead
+// of seven.
+template <class K, int G>
+__device__ __forceinline__ int teamSignedDistance(GroupCell<K, G>& w, bool act, unsigned box, double alphaI, d3 nI,
+                                                  double& dOut, d3& icOut, d3& isOut, uint32_t& err) {
+    constexpr int kGroups = 32 / G;
+    int st = 0;
+    unsigned above, under;
+    if (!groupLevels(w, act, box, alphaI, nI, st, above, under)) return st;  // (the whole warp)
+    const double* sv = w.sh->sv[w.g];
+    int lowLabel = 0, upLabel = w.np - 1;
+    unsigned known = 0;  // levels whose volume is known,
+    double vol = 0.0;    // that of level j on lane j
+    // moves (lo, up) past the clear levels; whether that ends the bisection
+    const auto fixed = [&](int& lo, int& up) {
+        while (up - lo > 1) {
+            const int mid = (up + lo + 1) >> 1;
+            if ((above >> mid) & 1u) up = mid;
+            else if ((under >> mid) & 1u) lo = mid;
+            else return false;
+        }
+        return true;
+    };
+    enum { kBisect, kCubic, kFinal };
+    int phase = kBisect;
+    unsigned tasks = 0;  // kCubic: 1, 2 the ends of the bracket, 4, 8 its thirds
+    Bracket br;
+    br.lowA = 0.0;
+    br.upA = 1.0;
+    br.lowD = br.upD = 0.0;
+    double v13 = 0.0, v23 = 0.0, deltaDistance = 0.0, distance = 0.0;
+    SubCell sc;
+    for (;;) {
+        bool want = false;
+        double d = 0.0;
+        int mine = -1;  // the group's level or task
+        if (phase == kBisect) {
+            bool found = false;
+            while (upLabel - lowLabel > 1) {
+                const int mid = (upLabel + lowLabel + 1) >> 1;
+                bool more;
+                if ((known >> mid) & 1u) {
+                    const double a = __shfl_sync(kAllLanes, vol, mid);
+                    if (absBelow(a - alphaI, kTSMALL)) {
+                        found = true;
+                        distance = sv[mid];
+                        break;
+                    }
+                    more = a > alphaI;
+                } else if ((above >> mid) & 1u) {
+                    more = true;
+                } else if ((under >> mid) & 1u) {
+                    more = false;
+                } else {
+                    break;
+                }
+                (more ? upLabel : lowLabel) = mid;
+            }
+            if (found) {
+                phase = kFinal;
+            } else if (upLabel - lowLabel > 1) {
+                // node g of the tree of levels that may be asked for
+                int lo = lowLabel, up = upLabel;
+                int bit = 31 - __clz(w.g + 1);
+                bool open = !fixed(lo, up);
+                for (--bit; bit >= 0 && open; --bit) {
+                    const int mid = (up + lo + 1) >> 1;
+                    (((w.g + 1) >> bit) & 1 ? lo : up) = mid;
+                    open = !fixed(lo, up);
+                }
+                want = open;
+                if (want) {
+                    mine = (up + lo + 1) >> 1;
+                    d = sv[mine];
+                }
+            } else {
+                br.lowD = sv[lowLabel];
+                br.upD = sv[upLabel];
+                deltaDistance = divByRecip(br.upD - br.lowD, 3.0, 1.0 / 3.0);
+                if (absBelow(br.lowD - br.upD, kTSMALL)) {  // levels that coincide: their middle
+                    distance = 0.5 * (br.lowD + br.upD);
+                    phase = kFinal;
+                } else {
+                    phase = kCubic;
+                    tasks = 12u;
+                    const double a = __shfl_sync(kAllLanes, vol, lowLabel), b = __shfl_sync(kAllLanes, vol, upLabel);
+                    if ((known >> lowLabel) & 1u) br.lowA = a;
+                    else if (lowLabel != 0) tasks |= 1u;
+                    if ((known >> upLabel) & 1u) br.upA = b;
+                    else if (upLabel != w.np - 1) tasks |= 2u;
+                }
+            }
+        }
+        if (phase == kCubic) {
+            unsigned t = tasks;
+            for (int k = 0; k < w.g; ++k) t &= t - 1u;
+            want = t != 0;
+            mine = want ? __ffs(t) - 1 : -1;
+            d = mine == 0 ? br.lowD : (mine == 1 ? br.upD : br.lowD + (mine == 2 ? deltaDistance : 2.0 * deltaDistance));
+        } else if (phase == kFinal) {
+            want = true;
+            d = distance;
+        }
+        groupSubCell(w, want, phase != kFinal, d, sc, err);
+        if (phase == kFinal) {
+            dOut = d;
+            icOut = sc.ic;
+            isOut = sc.is;
+            return sc.status;
+        }
+#pragma unroll
+        for (int k = 0; k < kGroups; ++k) {
+            const int q = __shfl_sync(kAllLanes, mine, k * G);
+            const double v = __shfl_sync(kAllLanes, sc.vof, k * G);
+            if (q < 0) continue;
+            if (phase == kBisect) {
+                known |= 1u << q;
+                if (w.lane == q) vol = v;
+            } else {
+                tasks &= ~(1u << q);
+                if (q == 0) br.lowA = v;
+                else if (q == 1) br.upA = v;
+                else if (q == 2) v13 = v;
+                else v23 = v;
+            }
+        }
+        if (phase == kCubic && tasks == 0) {
+            distance = cubicDistance(br, v13, v23, alphaI);
+            phase = kFinal;
+        }
+    }
 }
 
 }  // namespace simplic

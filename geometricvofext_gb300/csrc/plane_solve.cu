@@ -4,13 +4,13 @@
 //
 // One GB300, kernel time with one thread per cell -> a group per cell -> with
 // the work left out that plane_group.cuh lists (deformation field; interface
-// cells in brackets):
-//   24^3 hex (331) 0.861 -> 0.167 -> 0.101 ms
-//   33^3 hex (617) 0.880 -> 0.224 -> 0.138 ms
+// cells in brackets) -> a warp per cell on short lists:
+//   24^3 hex (331) 0.861 -> 0.167 -> 0.101 -> 0.049 ms
+//   33^3 hex (617) 0.880 -> 0.224 -> 0.138 -> 0.066 ms
 //   128^3 hex (30,189) 1.451 -> 1.345 -> 0.660 ms
 //   256^3 hex (35,452) 1.636 -> 1.628 -> 0.764 ms
 //   96^3 warped hex (7,146) 0.985 -> 0.406 -> 0.348 ms
-//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 -> 1.56 ms
+//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 -> 1.56 -> 1.24 ms
 // At the large sizes the FP64 pipe is about 80% busy.
 #include "plane_group.cuh"
 #include "simplic_kernels.h"
@@ -24,6 +24,15 @@ namespace {
 // Warps are independent, so a block is only the unit shared memory is handed
 // out in: two warps keep the largest workspace within the static limit.
 constexpr int kPlaneThreads = 64;
+
+// Lists of up to this many cells per SM leave FP64 pipes idle when the warps
+// are filled (four pipes an SM, busy half the time with one warp each): there a
+// warp takes one cell, a group a cut (teamSignedDistance).  Filled warps
+// against one cell each, ms: hexahedra 365 cells 0.105 / 0.055, 936 0.140 /
+// 0.069, 1,778 0.140 / 0.097, 2,296 0.113 / 0.131; warped hexahedra 387 0.158 /
+// 0.099, 1,054 0.215 / 0.181, 1,578 0.192 / 0.200; tetrahedra 560 0.120 /
+// 0.083, 1,131 0.122 / 0.123, 2,016 0.123 / 0.236.  152 SMs: the line is 1,216.
+constexpr int kTeamPerSm = 8;
 
 // One instantiation per cell class (workspace caps K, G lanes per cell); a
 // launch handles the mixed cells of its class.  With SPLIT the workspace is
@@ -47,8 +56,11 @@ __global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, Plane
     uint32_t err = 0;
     // warps are dealt out one per block before any block gets a second
     const int warps = gridDim.x * (kPlaneThreads / 32);
-    for (int q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; q * kCells < nm; q += warps) {
-        const int k = q * kCells + w.g;
+    const int first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const bool team = kCells > 1 && nm <= p.teamMax;
+    const int cells = team ? 1 : kCells;  // of a warp
+    for (int q = first; q * cells < nm; q += warps) {
+        const int k = team ? q : q * kCells + w.g;
         bool act = k < nm;
         const int i = act && p.rest ? p.rest[k] : k;
         const int c = act ? p.mixed[i] : 0;
@@ -68,12 +80,13 @@ __global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, Plane
         const double alphaI = act ? p.alpha[c] : 0.0;
         const d3 nI = act ? ld3(p.nrm, i) : mk(0, 0, 0);
         const unsigned box = (act && !SPLIT) ? m.boxCorner[c] : 0u;
-        int st = groupSignedDistance(w, act && ok, box, alphaI, nI, d, ic, is, err);
+        int st = team ? teamSignedDistance(w, act && ok, box, alphaI, nI, d, ic, is, err)
+                      : groupSignedDistance(w, act && ok, box, alphaI, nI, d, ic, is, err);
         if (act && !ok) {
             err |= kErrSubFaceOverflow;
             st = 1;
         }
-        if (act && w.l == 0) {
+        if (act && w.l == 0 && (!team || w.g == 0)) {
             p.mStatus[i] = int8_t(st);
             p.status[c] = int8_t(st);
             p.dOut[i] = d;
@@ -83,6 +96,13 @@ __global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, Plane
         __syncwarp();
     }
     if (err) atomicOr(p.err, err);
+}
+
+int smCount() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
 }
 
 // A grid of exactly the blocks that are resident at once on all SMs, looked
@@ -135,6 +155,7 @@ PlaneArgs planeArgs(const StepArgs& a) {
     p.err = a.err;
     p.skip = nullptr;
     p.rest = nullptr;
+    p.teamMax = kTeamPerSm * smCount();
     return p;
 }
 

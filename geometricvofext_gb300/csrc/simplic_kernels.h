@@ -135,6 +135,7 @@ struct PlaneArgs {
     double* isOut;
     uint32_t* err;
     const uint8_t* skip;  // optional per mixed cell: nonzero keeps the previous plane (isoRDF)
+    int teamMax;          // lists up to here: a warp per cell
     const int* rest;      // optional list of mixed positions to solve, *nMixed of them
 };
 

@@ -250,6 +250,17 @@ __device__ __forceinline__ bool absBelow(double x, double t) {  // fabs(x) < t, 
     return (bitsOf(x) & 0x7fffffffffffffffLL) < bitsOf(t);
 }
 
+// a double's leading 24 bits as a float (truncated), on the integer pipe;
+// zero below the float range, infinite above it
+__device__ __forceinline__ float leadingFloat(double x) {
+    const long long b = bitsOf(x);
+    const int e = int((b >> 52) & 0x7ff) - 896;
+    const unsigned s = unsigned(b >> 32) & 0x80000000u;
+    if (e <= 0) return __uint_as_float(s);
+    if (e >= 255) return __uint_as_float(s | 0x7f800000u);
+    return __uint_as_float(s | (unsigned(e) << 23) | (unsigned(b >> 29) & 0x7fffffu));
+}
+
 // Newton on the cubic through the bracket (cutCell.C:743-789); returns the
 // plane constant.
 __device__ __forceinline__ double cubicDistance(const Bracket& br, double v13, double v23, double alphaI) {

@@ -116,90 +116,347 @@ __device__ __forceinline__ d3 pointValue(const DevMesh& m, int p, const double* 
     return r;
 }
 
-// cell-point interpolation (the restatement documented in the oracle)
+struct F3 {
+    float x, y, z;
+};
+__device__ __forceinline__ F3 leadingF3(d3 v) { return {leadingFloat(v.x), leadingFloat(v.y), leadingFloat(v.z)}; }
+__device__ __forceinline__ F3 operator-(F3 a, F3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ float maxAbs(F3 a) { return fmaxf(fabsf(a.x), fmaxf(fabsf(a.y), fabsf(a.z))); }
+__device__ __forceinline__ float det3(F3 a, F3 b, F3 c) {
+    return a.x * (b.y * c.z - b.z * c.y) + a.y * (b.z * c.x - b.x * c.z) + a.z * (b.x * c.y - b.y * c.x);
+}
+
+// Bounds of the least weight of r in the tetrahedron.  The components are
+// differences of coordinates up to M cut to 24 bits, so each is within q =
+// 2^-21 M + 2^-22 L of the exact one (L the largest of them); a triple
+// product's error is below 18 L^2 q from the components and 30 2^-24 L^3 from
+// its own roundings, together below E = 32 L^2 q (the apex's, a sum of four: 4
+// E).  With |det| > 2 E a quotient w is then within 2 E (4 + |w|) / |det| and
+// the division's own error; the double weights are far closer.
+__device__ __forceinline__ void leastWeightBounds(F3 r, F3 e1, F3 e2, F3 e3, float M, float& lo, float& hi) {
+    const float L = fmaxf(fmaxf(maxAbs(r), maxAbs(e1)), fmaxf(maxAbs(e2), maxAbs(e3)));
+    const float E = 32.f * L * L * (0x1p-21f * M + 0x1p-22f * L);
+    const float det = det3(e1, e2, e3);
+    lo = -FLT_MAX;
+    hi = FLT_MAX;
+    if (!(E > 1e-30f && L < 1e9f && fabsf(det) > 2.f * E)) return;
+    const float y = 1.f / det;
+    const float n1 = det3(r, e2, e3), n2 = det3(e1, r, e3), n3 = det3(e1, e2, r);
+    const float n0 = ((det - n1) - n2) - n3;
+    const float w = fminf(fminf(n0 * y, n1 * y), fminf(n2 * y, n3 * y));
+    const float err = 2.f * E * (4.f + fabsf(w)) * fabsf(y) + 1e-6f * fabsf(w);
+    lo = w - err;
+    hi = w + err;
+}
+
+// U(x) in cell c by one thread: the cell-point interpolation (the restatement
+// documented in the oracle), the weights in the first of the cell's tetrahedra
+// (centre, fan triangle of a face) that holds x up to -1e-10, else in the one
+// with the largest least weight.  The search passes over the tetrahedra that
+// cannot hold x by their single precision bounds; if none holds it (cells of
+// warped faces), over those that cannot have the largest.
 __device__ __forceinline__ d3 interpolateU(const DevMesh& m, int c, d3 x, const double* U, const double* Ub) {
     const d3 a = ld3(m.C, c);
     const d3 r = x - a;
     int bp0 = -1, bp1 = -1, bp2 = -1;
-    double bw0 = 0, bw1 = 0, bw2 = 0, bw3 = 0, bestMin = -1e300;
+    double bw[4] = {0, 0, 0, 0}, bestMin = -1e300;
+    const int k1 = m.cOff[c + 1];
+    const F3 aF = leadingF3(a), rF = leadingF3(r);
+    const float aM = maxAbs(aF);
+    float most = -FLT_MAX;  // a lower bound of the largest least weight
     bool found = false;
-    for (int k = m.cOff[c]; k < m.cOff[c + 1] && !found; ++k) {
-        const int f = m.cFaces[k];
-        const int q0 = m.fOff[f], n = m.fOff[f + 1] - q0;
-        const int g0 = m.fPts[q0];
-        const d3 e1 = ld3(m.pts, g0) - a;
-        for (int i = 1; i + 1 < n; ++i) {
-            const int gi = m.fPts[q0 + i], gj = m.fPts[q0 + i + 1];
-            const d3 e2 = ld3(m.pts, gi) - a, e3 = ld3(m.pts, gj) - a;
-            const double det = dot(e1, cross(e2, e3));
+    for (int trip = 0; trip < 2 && !found; ++trip) {
+        bp0 = -1;
+        bestMin = -1e300;
+        int k = m.cOff[c], i = 0, n = 0, q0 = 0, g0 = 0;
+        F3 f1, f3;
+        while (!found) {
+            bool candidate = false;  // the next tetrahedron x may be in
+            while (true) {
+                if (i + 1 >= n) {
+                    if (k >= k1) break;
+                    const int f = m.cFaces[k++];
+                    q0 = m.fOff[f];
+                    n = m.fOff[f + 1] - q0;
+                    if (n < 3) {
+                        n = 0;
+                        continue;
+                    }
+                    i = 1;
+                    g0 = m.fPts[q0];
+                    f1 = leadingF3(ld3(m.pts, g0));
+                    f3 = leadingF3(ld3(m.pts, m.fPts[q0 + 1]));
+                }
+                const F3 f2 = f3;
+                f3 = leadingF3(ld3(m.pts, m.fPts[q0 + i + 1]));
+                ++i;
+                const float M = fmaxf(fmaxf(aM, maxAbs(f1)), fmaxf(maxAbs(f2), maxAbs(f3)));
+                float lo, hi;
+                leastWeightBounds(rF, f1 - aF, f2 - aF, f3 - aF, M, lo, hi);
+                if (trip == 0) most = fmaxf(most, lo);
+                candidate = !(hi < (trip == 0 ? -1e-9f : most));
+                if (candidate) break;
+            }
+            if (!candidate) break;
+            const int gi = m.fPts[q0 + i - 1], gj = m.fPts[q0 + i];
+            const d3 e1 = ld3(m.pts, g0) - a, e2 = ld3(m.pts, gi) - a, e3 = ld3(m.pts, gj) - a;
+            const d3 c23 = cross(e2, e3);
+            const double det = dot(e1, c23);
             if (!(fabs(det) > kVSMALL)) continue;
-            const double w1 = dot(r, cross(e2, e3)) / det;
-            const double w2 = dot(e1, cross(r, e3)) / det;
-            const double w3 = dot(e1, cross(e2, r)) / det;
-            const double w0 = ((1.0 - w1) - w2) - w3;
-            const double mn = fmin(fmin(w0, w1), fmin(w2, w3));
-            if (mn > bestMin || mn >= -1e-10) {
+            const d3 w = divBy(mk(dot(r, c23), dot(e1, cross(r, e3)), dot(e1, cross(e2, r))), det);
+            const double w0 = ((1.0 - w.x) - w.y) - w.z;
+            const double mn = fmin(fmin(w0, w.x), fmin(w.y, w.z));
+            found = mn >= -1e-10;
+            if (found || mn > bestMin) {
                 bestMin = mn;
                 bp0 = g0;
                 bp1 = gi;
                 bp2 = gj;
-                bw0 = w0;
-                bw1 = w1;
-                bw2 = w2;
-                bw3 = w3;
-            }
-            if (mn >= -1e-10) {
-                found = true;
-                break;
+                bw[0] = w0;
+                bw[1] = w.x;
+                bw[2] = w.y;
+                bw[3] = w.z;
             }
         }
     }
     if (bp0 < 0) return ld3(U, c);
-    d3 t = bw0 * ld3(U, c);
-    t = t + bw1 * pointValue(m, bp0, U, Ub);
-    t = t + bw2 * pointValue(m, bp1, U, Ub);
-    t = t + bw3 * pointValue(m, bp2, U, Ub);
+    d3 t = bw[0] * ld3(U, c);
+    t = t + bw[1] * pointValue(m, bp0, U, Ub);
+    t = t + bw[2] * pointValue(m, bp1, U, Ub);
+    t = t + bw[3] * pointValue(m, bp2, U, Ub);
     return t;
 }
 
-// (a) interface speed Un0 = U(interface centre) . n of every cut cell, and
+// (a) Interface speed Un0 = U(interface centre) . n of every cut cell, and
 //     the list of its downwind faces (advection.C:131-174: phi >= 0 on an
-//     owned face, phi < 0 on a neighboured one; boundary faces phi >= 0)
-__global__ void __launch_bounds__(128) kInterfaceUn0(DevMesh m, const int* __restrict__ mixed,
-                                                     const int* __restrict__ nMixed,
-                                                     const int8_t* __restrict__ mStatus,
-                                                     const double* __restrict__ nrm, const double* __restrict__ icArr,
-                                                     const double* __restrict__ U, const double* __restrict__ Ub,
-                                                     const double* __restrict__ phi, double* __restrict__ un0,
-                                                     int2* __restrict__ dwList, int* __restrict__ dwCount) {
+//     owned face, phi < 0 on a neighboured one; boundary faces phi >= 0).
+//
+// A thread per cell (interpolateU) is a chain of dependent loads and, with 32
+// cells a warp, of one or two tetrahedra at 80 FP64 instructions and the
+// points' sums at 144 (all twelve tetrahedra of a hexahedron before the single
+// precision bounds).  Lists that leave warps idle give a cell eight lanes, four
+// cells a warp:
+//   * on its faces, naming the first tetrahedron that may hold x;
+//   * on that one's determinant and three numerators, the same triple product
+//     with one vector each replaced by x;
+//   * on the points' cells (velocity times weight), then on the nine sums over
+//     them in order; on the faces again for the list.
+// That is 70 to 100 FP64 instructions for four cells: more of the pipe per
+// cell, which decides beyond kUn0Group cells per SM.
+// Kernel time of the walk in double -> a thread per cell with the bounds ->
+// eight lanes: 24^3 hexahedra (331 cells) 66 -> 38 -> 20 us, 33^3 (617) 65 -> 44
+// -> 29, 112^3 (6,988) - -> 74 -> 54, 128^3 (30,189) 107 -> 81 -> 104, 256^3
+// (35,452) 118 -> 95 -> 128, warped 96^3 (7,146) 67 -> 79 -> 51, refined 24^3
+// (755) 201 -> 90 -> 43.  The two lines meet near 100 cells per SM.
+constexpr int kUn0Group = 96;
+constexpr int kUn0Threads = 128;
+__global__ void __launch_bounds__(kUn0Threads) kInterfaceUn0(
+    DevMesh m, const int* __restrict__ mixed, const int* __restrict__ nMixed, const int8_t* __restrict__ mStatus,
+    const double* __restrict__ nrm, const double* __restrict__ icArr, const double* __restrict__ U,
+    const double* __restrict__ Ub, const double* __restrict__ phi, double* __restrict__ un0,
+    int2* __restrict__ dwList, int* __restrict__ dwCount, int groupMax) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kNone = INT_MAX;
+    __shared__ double prodS[kUn0Threads / 32][4][9][9];  // (row padded) [point, component][cell of the chunk]
+    const int lane = threadIdx.x & 31, l = lane & 7, g = lane >> 3, base = lane & 24;
+    double(*prod)[9] = prodS[threadIdx.x >> 5][g];
     const int nm = *nMixed;
-    const int lane = threadIdx.x & 31;
-    // uniform trip count per warp so the list append can use warp shuffles
-    const int stride = spreadStride();
-    const int nIter = (nm + stride - 1) / stride;
-    for (int it = 0; it < nIter; ++it) {
-        const int i = it * stride + spreadFirst();
-        int nd = 0, k0 = 0;
-        unsigned down = 0;  // bit j: the cell's j-th face (cells() order) is downwind
-        if (i < nm && mStatus[i] == 0) {
-            const int c = mixed[i];
-            un0[i] = dot(interpolateU(m, c, ld3(icArr, i), U, Ub), ld3(nrm, i));
-            k0 = m.cOff[c];
-            down = downwindFaces(m, c, k0, m.cOff[c + 1], phi);
-            nd = __popc(down);
+    if (nm > groupMax) {
+        // uniform trip count per warp so the list append can use warp shuffles
+        const int stride = spreadStride();
+        const int nIter = (nm + stride - 1) / stride;
+        for (int it = 0; it < nIter; ++it) {
+            const int i = it * stride + spreadFirst();
+            int nd = 0, k0 = 0;
+            unsigned down = 0;  // bit j: the cell's j-th face (cells() order) is downwind
+            if (i < nm && mStatus[i] == 0) {
+                const int c = mixed[i];
+                un0[i] = dot(interpolateU(m, c, ld3(icArr, i), U, Ub), ld3(nrm, i));
+                k0 = m.cOff[c];
+                down = downwindFaces(m, c, k0, m.cOff[c + 1], phi);
+                nd = __popc(down);
+            }
+            // warp-aggregated append
+            int incl = nd;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            int base = 0;
+            if (lane == 31 && total) base = atomicAdd(dwCount, total);
+            base = __shfl_sync(0xffffffffu, base, 31);
+            int q = base + incl - nd;
+            for (unsigned mm = down; mm; mm &= mm - 1u) dwList[q++] = make_int2(i, m.cFaces[k0 + __ffs(mm) - 1]);
         }
-        // warp-aggregated append
-        int incl = nd;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
+        return;
+    }
+    constexpr int kCells = kUn0Threads / 8;  // of a block
+    __shared__ int listS[2];  // entries of the block's cells in the list, where they start
+    for (int q = blockIdx.x; q * kCells < nm; q += gridDim.x) {
+        const int i = q * kCells + 4 * (threadIdx.x >> 5) + g;
+        if (threadIdx.x == 0) listS[0] = 0;
+        __syncthreads();
+        const bool act = i < nm && mStatus[i] == 0;
+        const int c = act ? mixed[i] : 0;
+        const int k0 = act ? m.cOff[c] : 0, k1 = act ? m.cOff[c + 1] : 0;
+        const d3 a = ld3(m.C, c);
+        const d3 x = act ? ld3(icArr, i) : a;
+        const F3 aF = leadingF3(a), rF = leadingF3(x - a);
+        const float aM = maxAbs(aF);
+        const int l3 = l < 3 ? l : 0;  // component l on lanes 0-2
+        const double uC = U[size_t(3) * c + l3], nI = act ? nrm[size_t(3) * i + l3] : 0.0;
+        // the downwind faces: one addition to the list's length per block,
+        // whose answer is read at the end
+        const auto downwind = [&](int k) {
+            if (k >= k1) return false;
+            const int f = m.cFaces[k];
+            const long long ph = bitsOf(phi[f]);
+            const bool owned = f >= m.nfi || m.own[f] == c;
+            return owned ? nonNegBits(ph) : (!nonNegBits(ph) && (ph & 0x7fffffffffffffffLL) <= 0x7ff0000000000000LL);
+        };
+        unsigned down = 0;  // bit j: the lane's j-th face, l + 8 j
+        for (int j = 0; k0 + l + 8 * j < k1; ++j) down |= unsigned(downwind(k0 + l + 8 * j)) << j;
+        int mine = 0;
+        if (down) mine = atomicAdd(&listS[0], __popc(down));
+        __syncthreads();
+        if (threadIdx.x == 0) listS[1] = listS[0] ? atomicAdd(dwCount, listS[0]) : 0;
+        // the tetrahedron
+        int bp[3] = {-1, -1, -1};
+        double bw[4] = {0, 0, 0, 0}, bestMin = -1e300;
+        bool open = act, any = false;  // any: the second trip, for the largest weight
+        int from = 0;                  // tetrahedra (16 face + triangle) from here on
+        float most = -FLT_MAX;         // a lower bound of the largest least weight
+        while (__any_sync(kAll, open)) {
+            const float least = any ? most : -1e-9f;
+            int cand = kNone;
+            float low = -FLT_MAX;
+            for (int k = k0 + l; open && k < k1; k += 8) {
+                const int f = m.cFaces[k];
+                const int q0 = m.fOff[f], n = m.fOff[f + 1] - q0;
+                if (n < 3) continue;
+                const F3 f1 = leadingF3(ld3(m.pts, m.fPts[q0]));
+                F3 f3 = leadingF3(ld3(m.pts, m.fPts[q0 + 1]));
+                for (int t = 1; t + 1 < n; ++t) {
+                    const F3 f2 = f3;
+                    f3 = leadingF3(ld3(m.pts, m.fPts[q0 + t + 1]));
+                    const float M = fmaxf(fmaxf(aM, maxAbs(f1)), fmaxf(maxAbs(f2), maxAbs(f3)));
+                    float lo, hi;
+                    leastWeightBounds(rF, f1 - aF, f2 - aF, f3 - aF, M, lo, hi);
+                    low = fmaxf(low, lo);
+                    const int id = 16 * (k - k0) + t;
+                    if (id >= from && id < cand && !(hi < least)) cand = id;
+                }
+            }
+            for (int o = 4; o; o >>= 1) {
+                cand = min(cand, __shfl_xor_sync(kAll, cand, o));
+                low = fmaxf(low, __shfl_xor_sync(kAll, low, o));
+            }
+            if (open) most = low;
+            if (cand == kNone) {  // none (left): the second trip, or the end
+                open = open && !any;
+                if (open) {
+                    any = true;
+                    from = 0;
+                    bp[0] = -1;
+                    bestMin = -1e300;
+                }
+            }
+            const bool eval = cand != kNone;
+            int gp[3] = {0, 0, 0};
+            if (eval) {
+                const int q0 = m.fOff[m.cFaces[k0 + (cand >> 4)]], t = cand & 15;
+                gp[0] = m.fPts[q0];
+                gp[1] = m.fPts[q0 + t];
+                gp[2] = m.fPts[q0 + t + 1];
+                from = cand + 1;
+            }
+            const d3 u = ((l & 3) == 1 ? x : ld3(m.pts, gp[0])) - a, v = ((l & 3) == 2 ? x : ld3(m.pts, gp[1])) - a,
+                     w = ((l & 3) == 3 ? x : ld3(m.pts, gp[2])) - a;
+            const double tri = dot(u, cross(v, w));
+            const double det = __shfl_sync(kAll, tri, base);
+            const double quot = tri / det;
+            const double w1 = __shfl_sync(kAll, quot, base + 1), w2 = __shfl_sync(kAll, quot, base + 2),
+                         w3 = __shfl_sync(kAll, quot, base + 3);
+            const double w0 = ((1.0 - w1) - w2) - w3;
+            const double mn = fmin(fmin(w0, w1), fmin(w2, w3));
+            if (eval && fabs(det) > kVSMALL) {
+                open = !(mn >= -1e-10);
+                if (!open || mn > bestMin) {
+                    bestMin = mn;
+                    bp[0] = gp[0];
+                    bp[1] = gp[1];
+                    bp[2] = gp[2];
+                    bw[0] = w0;
+                    bw[1] = w1;
+                    bw[2] = w2;
+                    bw[3] = w3;
+                }
+            }
         }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        int base = 0;
-        if (lane == 31 && total) base = atomicAdd(dwCount, total);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        int q = base + incl - nd;
-        for (unsigned mm = down; mm; mm &= mm - 1u) dwList[q++] = make_int2(i, m.cFaces[k0 + __ffs(mm) - 1]);
+        // the values at its points: sum k = 3 point + component on lane k, the
+        // ninth on lane 0 too
+        const bool tet = act && bp[0] >= 0;
+        int at[3], end[3];
+        bool boundary[3];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            const int pt = tet ? bp[p] : 0;
+            const int b0 = m.pbOff[pt], b1 = m.pbOff[pt + 1], c0 = m.pcOff[pt], c1 = m.pcOff[pt + 1];
+            boundary[p] = b1 > b0;
+            at[p] = boundary[p] ? b0 : c0;
+            end[p] = tet ? (boundary[p] ? b1 : c1) : at[p];
+        }
+        double sum = 0.0, sum8 = 0.0;
+        while (__any_sync(kAll, at[0] < end[0] || at[1] < end[1] || at[2] < end[2])) {
+            int id[3];
+            double wt[3];
+            bool in[3];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                const int k = at[p] + l;
+                in[p] = k < end[p];
+                id[p] = in[p] ? (boundary[p] ? m.pbFaces : m.pCells)[k] : 0;
+                wt[p] = in[p] ? (boundary[p] ? m.pbW : m.pcW)[k] : 0.0;
+            }
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                const double* row = U;
+                if (in[p]) {
+                    if (!boundary[p]) row = U + size_t(3) * id[p];
+                    else row = Ub ? Ub + size_t(3) * (id[p] - m.nfi) : U + size_t(3) * m.own[id[p]];
+                }
+                prod[3 * p][l] = wt[p] * row[0];
+                prod[3 * p + 1][l] = wt[p] * row[1];
+                prod[3 * p + 2][l] = wt[p] * row[2];
+            }
+            __syncwarp();
+            const int n01 = (l < 3 ? end[0] - at[0] : (l < 6 ? end[1] - at[1] : end[2] - at[2]));
+            const int n8 = l == 0 ? end[2] - at[2] : 0;
+            for (int j = 0; j < 8; ++j) {
+                if (j < n01) sum = sum + prod[l][j];
+                if (j < n8) sum8 = sum8 + prod[8][j];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < 3; ++p) at[p] = min(at[p] + 8, end[p]);
+        }
+        // U(x) by components, and its part of Un0
+        double t = uC;
+        const double v0 = __shfl_sync(kAll, sum, base + l3), v1 = __shfl_sync(kAll, sum, base + 3 + l3);
+        double v2 = __shfl_sync(kAll, sum, base + 6 + (l3 & 1));
+        const double v8 = __shfl_sync(kAll, sum8, base);
+        if (l3 == 2) v2 = v8;
+        if (tet) t = ((bw[0] * t + bw[1] * v0) + bw[2] * v1) + bw[3] * v2;
+        const double part = t * nI;
+        const double px = __shfl_sync(kAll, part, base), py = __shfl_sync(kAll, part, base + 1),
+                     pz = __shfl_sync(kAll, part, base + 2);
+        if (act && l == 0) un0[i] = (px + py) + pz;
+        __syncthreads();
+        int dst = listS[1] + mine;
+        for (unsigned mm = down; mm; mm &= mm - 1u)
+            dwList[dst++] = make_int2(i, m.cFaces[k0 + l + 8 * (__ffs(mm) - 1)]);
+        __syncthreads();
     }
 }
 
@@ -675,8 +932,9 @@ void launchLsNormal(const StepArgs& a, cudaStream_t st) {
 }
 
 void launchInterfaceUn0(const StepArgs& a, cudaStream_t st) {
-    kInterfaceUn0<<<residentGrid(kInterfaceUn0, 128), 128, 0, st>>>(a.m, a.mixed, a.nMixed, a.mStatus, a.nrm, a.icArr, a.U, a.Ub,
-                                                      a.phi, a.un0, a.dwList, a.dwCount);
+    kInterfaceUn0<<<residentGrid(kInterfaceUn0, kUn0Threads), kUn0Threads, 0, st>>>(
+        a.m, a.mixed, a.nMixed, a.mStatus, a.nrm, a.icArr, a.U, a.Ub, a.phi, a.un0, a.dwList, a.dwCount,
+        kUn0Group * smCount());
 }
 
 template <bool WARPED>

@@ -99,17 +99,6 @@ __device__ __forceinline__ double halfOf(double x) {
     return 0.5 * x;
 }
 
-// a double's leading 24 bits as a float (truncated), on the integer pipe;
-// zero below the float range, infinite above it
-__device__ __forceinline__ float leadingFloat(double x) {
-    const long long b = bitsOf(x);
-    const int e = int((b >> 52) & 0x7ff) - 896;
-    const unsigned s = unsigned(b >> 32) & 0x80000000u;
-    if (e <= 0) return __uint_as_float(s);
-    if (e >= 255) return __uint_as_float(s | 0x7f800000u);
-    return __uint_as_float(s | (unsigned(e) << 23) | (unsigned(b >> 29) & 0x7fffffu));
-}
-
 // dot(a, b) >= 0 for the double-precision dot: the sign of a single
 // precision estimate where it is certain (each product is within 2^-21 of
 // the exact one, the estimate's sums within 2^-22 of the terms' magnitudes,

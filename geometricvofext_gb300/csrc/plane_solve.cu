@@ -98,13 +98,6 @@ __global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, Plane
     if (err) atomicOr(p.err, err);
 }
 
-int smCount() {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 1;
-}
-
 // A grid of exactly the blocks that are resident at once on all SMs, looked
 // up once per kernel and device.
 template <class Kernel>
@@ -140,6 +133,13 @@ void launchClass(const DevMesh& m, const PlaneArgs& p, int cls, cudaStream_t st)
 }
 
 }  // namespace
+
+int smCount() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
 
 PlaneArgs planeArgs(const StepArgs& a) {
     PlaneArgs p;

@@ -154,6 +154,7 @@ struct RdfBuffers {
     int stamp;
 };
 
+int smCount();  // of the current device
 void launchScanMixed(const StepArgs& a, cudaStream_t st);
 // isoRDF: band, cell -> mixed position map, alpha gradient (start); then per
 // iteration: normals from the gradient, the plane solve of the cells not

@@ -11,7 +11,7 @@
 //  K7 bruteForce         applyBruteForceBounding         advection.C:291-308
 //  faceFlatness          reconstruction::updateFaceFlatness reconstruction.C:408-440
 #include "face_group.cuh"
-#include "ls_fp64.cuh"
+#include "ls_group.cuh"
 #include "plain_geom.cuh"
 #include "simplic_kernels.h"
 
@@ -86,9 +86,25 @@ __global__ void __launch_bounds__(256) kScanMixed(int nc, const double* __restri
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) kLsNormal(DevMesh m, const double* __restrict__ alpha,
                                                  const int* __restrict__ mixed, const int* __restrict__ nMixed,
-                                                 double* __restrict__ nrm, uint32_t* __restrict__ errOut) {
+                                                 double* __restrict__ nrm, int groupMax,
+                                                 uint32_t* __restrict__ errOut) {
     const int nm = *nMixed;
     uint32_t err = 0;
+    if (nm <= groupMax) {
+        __shared__ LsRows rows[8];
+        const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+        for (int q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; 2 * q < nm; q += warps) {
+            const int i = 2 * q + (lane >> 4);
+            const bool act = i < nm;
+            const d3 g = groupLsGradient(m, act, act ? mixed[i] : 0, alpha, rows[threadIdx.x >> 4], err);
+            const d3 n = (-1.0) * g;
+            const int k = lane & 15;
+            const double s = mag(n) + kSMALL, v = (k == 0 ? n.x : (k == 1 ? n.y : n.z)) / s;
+            if (act && k < 3) nrm[size_t(3) * i + k] = v;
+        }
+        if (err) atomicOr(errOut, err);
+        return;
+    }
     for (int i = spreadFirst(); i < nm; i += spreadStride()) {
         const int c = mixed[i];
         const d3 g = lsGradientField(m, c, alpha, err);
@@ -928,7 +944,8 @@ void launchScanMixed(const StepArgs& a, cudaStream_t st) {
 }
 
 void launchLsNormal(const StepArgs& a, cudaStream_t st) {
-    kLsNormal<<<residentGrid(kLsNormal, 128), 128, 0, st>>>(a.m, a.aCur, a.mixed, a.nMixed, a.nrm, a.err);
+    kLsNormal<<<residentGrid(kLsNormal, 128), 128, 0, st>>>(a.m, a.aCur, a.mixed, a.nMixed, a.nrm,
+                                                            kLsGroup * smCount(), a.err);
 }
 
 void launchInterfaceUn0(const StepArgs& a, cudaStream_t st) {

@@ -10,7 +10,8 @@
 //   128^3 hex (30,189) 1.451 -> 1.345 -> 0.660 ms
 //   256^3 hex (35,452) 1.636 -> 1.628 -> 0.764 ms
 //   96^3 warped hex (7,146) 0.985 -> 0.406 -> 0.348 ms
-//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 -> 1.56 -> 1.24 ms
+//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 -> 1.56 -> 1.24 ms,
+//   then 0.71 with the classes in one launch
 // At the large sizes the FP64 pipe is about 80% busy.
 #include "plane_group.cuh"
 #include "simplic_kernels.h"
@@ -34,15 +35,12 @@ constexpr int kPlaneThreads = 64;
 // 0.083, 1,131 0.122 / 0.123, 2,016 0.123 / 0.236.  152 SMs: the line is 1,216.
 constexpr int kTeamPerSm = 8;
 
-// One instantiation per cell class (workspace caps K, G lanes per cell); a
-// launch handles the mixed cells of its class.  With SPLIT the workspace is
-// the splitWarpedFace one.
-// Six blocks per SM (168 registers, a few spilled) against four (200
-// registers): 0.80 against 0.82 ms at 128^3, 0.35 against 0.44 on the warped
-// 96^3 mesh; eight blocks spill more and gain nothing.
+// The mixed cells of one class (workspace caps K, G lanes per cell) on the
+// blocks first, first + 1 .. of a grid of `blocks`.  With SPLIT the workspace
+// is the splitWarpedFace one.
 template <class K, int G, bool SPLIT>
-__global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, PlaneArgs p, int cls) {
-    __shared__ GroupShared<K, G> shared[kPlaneThreads / 32];
+__device__ __forceinline__ void solveClass(const DevMesh& m, const PlaneArgs& p, int cls, GroupShared<K, G>* shared,
+                                           int block, int blocks) {
     constexpr int kCells = 32 / G;
     const int nm = *p.nMixed;
     const int mask = SPLIT ? m.splitClassMask : m.classMask;
@@ -55,8 +53,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, Plane
     w.l = w.lane - w.base;  // >= G on the lanes left over
     uint32_t err = 0;
     // warps are dealt out one per block before any block gets a second
-    const int warps = gridDim.x * (kPlaneThreads / 32);
-    const int first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const int warps = blocks * (kPlaneThreads / 32);
+    const int first = (threadIdx.x >> 5) * blocks + block;
     const bool team = kCells > 1 && nm <= p.teamMax;
     const int cells = team ? 1 : kCells;  // of a warp
     for (int q = first; q * cells < nm; q += warps) {
@@ -96,6 +94,41 @@ __global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, Plane
         __syncwarp();
     }
     if (err) atomicOr(p.err, err);
+}
+
+// Six blocks per SM (168 registers, a few spilled) against four (200
+// registers): 0.80 against 0.82 ms at 128^3, 0.35 against 0.44 on the warped
+// 96^3 mesh; eight blocks spill more and gain nothing.
+template <class K, int G, bool SPLIT>
+__global__ void __launch_bounds__(kPlaneThreads, 6) kPlaneSolve(DevMesh m, PlaneArgs p, int cls) {
+    __shared__ GroupShared<K, G> shared[kPlaneThreads / 32];
+    solveClass<K, G, SPLIT>(m, p, cls, shared, blockIdx.x, gridDim.x);
+}
+
+// Meshes with cells of several classes: a set of blocks for each, the largest
+// cells (the longest chains) first; the blocks of a class that has few cells
+// leave at once and the next take their place.  With one launch per class the
+// classes waited for one another: 24^3 of two sizes in a checkerboard (748
+// cells) 0.41 -> 0.24 ms, 36^3 (1,755) 0.71 -> 0.44, 48^3 (2,953) 0.69 -> 0.48,
+// 32^3 refined in the middle (1,423) 0.30 -> 0.21.
+template <bool SPLIT>
+__global__ void __launch_bounds__(kPlaneThreads, 5) kPlaneSolveAll(DevMesh m, PlaneArgs p, int mask, int blocks) {
+    constexpr int kWarps = kPlaneThreads / 32;
+    constexpr size_t kHex = sizeof(GroupShared<CapsHex, 6>), kPoly = sizeof(GroupShared<CapsPoly, 16>),
+                     kBig = sizeof(GroupShared<CapsBig, 32>), kMax = kHex > kPoly ? kHex : kPoly;
+    __shared__ __align__(16) unsigned char shared[kWarps * (kMax > kBig ? kMax : kBig)];
+    int set = blockIdx.x / blocks;
+    const int block = blockIdx.x - set * blocks;
+    for (int cls = 2; cls >= 0; --cls) {
+        if (!((mask >> cls) & 1) || set-- != 0) continue;
+        if (cls == 2)
+            solveClass<CapsBig, 32, SPLIT>(m, p, 2, reinterpret_cast<GroupShared<CapsBig, 32>*>(shared), block, blocks);
+        else if (cls == 1)
+            solveClass<CapsPoly, 16, SPLIT>(m, p, 1, reinterpret_cast<GroupShared<CapsPoly, 16>*>(shared), block,
+                                            blocks);
+        else
+            solveClass<CapsHex, 6, SPLIT>(m, p, 0, reinterpret_cast<GroupShared<CapsHex, 6>*>(shared), block, blocks);
+    }
 }
 
 // A grid of exactly the blocks that are resident at once on all SMs, looked
@@ -159,20 +192,23 @@ PlaneArgs planeArgs(const StepArgs& a) {
     return p;
 }
 
-static void launchAll(const StepArgs& a, const PlaneArgs& p, cudaStream_t st) {
-    // lanes per cell: the faces of the class (6 of hexahedra: five cells a
-    // warp; 12 of polyhedra on a half-warp; the whole warp beyond)
-    if (a.m.splitClassMask) {
-        const int mk = a.m.splitClassMask;
-        if (mk & 1) launchClass<CapsHex, 6, true>(a.m, p, 0, st);
-        if (mk & 2) launchClass<CapsPoly, 16, true>(a.m, p, 1, st);
-        if (mk & 4) launchClass<CapsBig, 32, true>(a.m, p, 2, st);
+// lanes per cell: the faces of the class (6 of hexahedra: five cells a warp;
+// 12 of polyhedra on a half-warp; the whole warp beyond)
+template <bool SPLIT>
+static void launchClasses(const DevMesh& m, const PlaneArgs& p, int mask, cudaStream_t st) {
+    if (mask & (mask - 1)) {
+        const int blocks = residentGrid(kPlaneSolveAll<SPLIT>), sets = (mask & 1) + ((mask >> 1) & 1) + ((mask >> 2) & 1);
+        kPlaneSolveAll<SPLIT><<<sets * blocks, kPlaneThreads, 0, st>>>(m, p, mask, blocks);
         return;
     }
-    const int mk = a.m.classMask;
-    if (mk & 1) launchClass<CapsHex, 6, false>(a.m, p, 0, st);
-    if (mk & 2) launchClass<CapsPoly, 16, false>(a.m, p, 1, st);
-    if (mk & 4) launchClass<CapsBig, 32, false>(a.m, p, 2, st);
+    if (mask & 1) launchClass<CapsHex, 6, SPLIT>(m, p, 0, st);
+    if (mask & 2) launchClass<CapsPoly, 16, SPLIT>(m, p, 1, st);
+    if (mask & 4) launchClass<CapsBig, 32, SPLIT>(m, p, 2, st);
+}
+
+static void launchAll(const StepArgs& a, const PlaneArgs& p, cudaStream_t st) {
+    if (a.m.splitClassMask) launchClasses<true>(a.m, p, a.m.splitClassMask, st);
+    else launchClasses<false>(a.m, p, a.m.classMask, st);
 }
 
 void launchPlaneSolve(const StepArgs& a, cudaStream_t st) { launchAll(a, planeArgs(a), st); }

@@ -840,21 +840,47 @@ __device__ __forceinline__ bool groupLevels(GroupCell<K, G>& w, bool act, unsign
     // (lane l on level l + 1).
     above = under = 0;
     const double* sv = s.sv[w.g];
+    bool up = false, dn = false;
+    float Lx = 0.f, Ly = 0.f, Lz = 0.f, far = 0.f;
     if (K::kFaces == 6) {
-        bool up = false, dn = false;
         if (act && box && l < 6) {
             const double *pl = s.P[w.g][(box >> 3) & 7], *ph = s.P[w.g][box & 7];
-            const float Lx = leadingFloat(ph[0] - pl[0]), Ly = leadingFloat(ph[1] - pl[1]),
-                        Lz = leadingFloat(ph[2] - pl[2]);
-            float far = 0.f;
+            Lx = leadingFloat(ph[0] - pl[0]);
+            Ly = leadingFloat(ph[1] - pl[1]);
+            Lz = leadingFloat(ph[2] - pl[2]);
             for (int k = 0; k < 3; ++k) far = fmaxf(far, fabsf(leadingFloat(pl[k])) + fabsf(leadingFloat(ph[k])));
-            if (fminf(Lx, fminf(Ly, Lz)) > 1e-8f * far)
-                levelEstimate(nI, Lx, Ly, Lz, leadingFloat(sv[0] - sv[7]), leadingFloat(sv[0] - sv[l + 1]),
-                              leadingFloat(alphaI), leadingFloat(1.0 - alphaI), up, dn);
         }
-        above = w.groupBits(__ballot_sync(kAllLanes, up)) << 1;
-        under = w.groupBits(__ballot_sync(kAllLanes, dn)) << 1;
+    } else if (__any_sync(kAllLanes, act && box)) {
+        // A cell that fills its bounding box up to 1e-6 of its volume (refined
+        // boxes, faces and edges split) cuts like the box, inside the margins:
+        // kernel on a 24^3 checkerboard 0.24 -> 0.165 ms, 56^3 0.73 -> 0.49.
+        static_assert(K::kFaces == 6 || K::kPts <= G, "a lane per point");
+        float lo[3], hi[3];
+        for (int k = 0; k < 3; ++k) {
+            const double p0 = act ? s.P[w.g][0][k] : 0.0, p = l < np ? s.P[w.g][l][k] : p0;
+            lo[k] = hi[k] = leadingFloat(p - p0);
+            far = fmaxf(far, 2.f * fabsf(leadingFloat(p)));
+        }
+        for (int o = G / 2; o; o >>= 1) {
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = fminf(lo[k], __shfl_xor_sync(kAllLanes, lo[k], o));
+                hi[k] = fmaxf(hi[k], __shfl_xor_sync(kAllLanes, hi[k], o));
+            }
+            far = fmaxf(far, __shfl_xor_sync(kAllLanes, far, o));
+        }
+        const float V = act ? leadingFloat(w.V) : 0.f;
+        const float B = (hi[0] - lo[0]) * (hi[1] - lo[1]) * (hi[2] - lo[2]);
+        if (act && box && fabsf(B - V) <= 1e-6f * V) {
+            Lx = hi[0] - lo[0];
+            Ly = hi[1] - lo[1];
+            Lz = hi[2] - lo[2];
+        }
     }
+    if (act && l < np - 2 && fminf(Lx, fminf(Ly, Lz)) > 1e-8f * far)
+        levelEstimate(nI, Lx, Ly, Lz, leadingFloat(sv[0] - sv[np - 1]), leadingFloat(sv[0] - sv[l + 1]),
+                      leadingFloat(alphaI), leadingFloat(1.0 - alphaI), up, dn);
+    above = w.groupBits(__ballot_sync(kAllLanes, up)) << 1;
+    under = w.groupBits(__ballot_sync(kAllLanes, dn)) << 1;
     return act;
 }
 

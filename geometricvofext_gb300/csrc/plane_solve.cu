@@ -11,7 +11,8 @@
 //   256^3 hex (35,452) 1.636 -> 1.628 -> 0.764 ms
 //   96^3 warped hex (7,146) 0.985 -> 0.406 -> 0.348 ms
 //   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 -> 1.56 -> 1.24 ms,
-//   then 0.71 with the classes in one launch
+//   then 0.71 with the classes in one launch, 0.49 with their boxes' levels
+//   settled in single precision
 // At the large sizes the FP64 pipe is about 80% busy.
 #include "plane_group.cuh"
 #include "simplic_kernels.h"
@@ -77,7 +78,8 @@ __device__ __forceinline__ void solveClass(const DevMesh& m, const PlaneArgs& p,
         d3 ic = mk(0, 0, 0), is = mk(0, 0, 0);
         const double alphaI = act ? p.alpha[c] : 0.0;
         const d3 nI = act ? ld3(p.nrm, i) : mk(0, 0, 0);
-        const unsigned box = (act && !SPLIT) ? m.boxCorner[c] : 0u;
+        // (of the classes beyond hexahedra any cell may be a box)
+        const unsigned box = (act && !SPLIT) ? (K::kFaces == 6 ? m.boxCorner[c] : 1u) : 0u;
         int st = team ? teamSignedDistance(w, act && ok, box, alphaI, nI, d, ic, is, err)
                       : groupSignedDistance(w, act && ok, box, alphaI, nI, d, ic, is, err);
         if (act && !ok) {

@@ -21,6 +21,7 @@
 #include "plain_geom.cuh"
 #include "simplic_kernels.h"
 
+#include <climits>
 #include <mutex>
 
 namespace simplic {
@@ -58,11 +59,75 @@ struct KahanV {
 // ---------------------------------------------------------------------------
 // normals: FP32 least squares
 // ---------------------------------------------------------------------------
+// On shorter lists 16 lanes take a cell, two cells a warp: a lane per stencil
+// cell for the loads and the FP64 differences, a lane per sum of the normal
+// equations (the same fused operations in the same order), one lane for the
+// elimination.  Kernel time, a thread per cell against 16 lanes: hexahedra 365
+// cells 22 / 9 us, 12,394 31 / 18, 30,189 31 / 27, 60,750 38 / 47; tetrahedra
+// 6,299 53 / 16.
+constexpr int kLsMixedGroup = 240;  // cells per SM
 __global__ void __launch_bounds__(128) kLsNormalMixed(DevMesh m, const double* __restrict__ alpha,
                                                       const int* __restrict__ mixed, const int* __restrict__ nMixed,
-                                                      double* __restrict__ nrm, uint32_t* __restrict__ errOut) {
+                                                      double* __restrict__ nrm, int groupMax,
+                                                      uint32_t* __restrict__ errOut) {
     const int nm = *nMixed;
     uint32_t err = 0;
+    if (nm <= groupMax) {
+        __shared__ float entS[8][16][5];  // of a cell: 1, x, y, z, alpha of 16 stencil cells; then its sums
+        const int lane = threadIdx.x & 31, l = lane & 15, r = l >> 2, q4 = l & 3;
+        float(*ent)[5] = entS[threadIdx.x >> 4];
+        const bool upper = r <= q4;
+        // factors of the lane's sum: A[r][q] on and above the diagonal, b[0..3]
+        // on lanes 4, 8, 12, 9
+        const int ia = upper ? r : (l == 9 ? 3 : r - 1), ib = upper ? q4 : 4;
+        const int warps = gridDim.x * (blockDim.x >> 5);
+        for (int q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; 2 * q < nm; q += warps) {
+            const int i = 2 * q + (lane >> 4);
+            const bool act = i < nm;
+            const int c = act ? mixed[i] : 0;
+            const int32_t* st = nullptr;
+            const int n = act ? stencilOf(m, c, st, err) + 1 : 0;
+            const int nMax = max(n, __shfl_xor_sync(0xffffffffu, n, 16));
+            const d3 Cc = ld3(m.C, c);
+            const double ac = alpha[c];
+            const float invH = rcbrtf(float(m.V[c]));
+            float acc = 0.f;
+            for (int e0 = 0; e0 < nMax; e0 += 16) {
+                const int e = e0 + l;
+                if (e < n) {
+                    const int x = e ? st[e - 1] : c;
+                    const d3 dx = ld3(m.C, x) - Cc;
+                    ent[l][0] = 1.f;
+                    ent[l][1] = float(dx.x) * invH;
+                    ent[l][2] = float(dx.y) * invH;
+                    ent[l][3] = float(dx.z) * invH;
+                    ent[l][4] = float(alpha[x] - ac);
+                }
+                __syncwarp();
+                const int top = min(16, nMax - e0);
+                for (int j = 0; j < top; ++j)
+                    if (e0 + j < n) acc = fmaf(ent[j][ia], ent[j][ib], acc);
+                __syncwarp();
+            }
+            float* sums = &ent[0][0];
+            sums[l] = acc;
+            __syncwarp();
+            if (act && l == 0) {
+                float A[4][4], b[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                    for (int j = k; j < 4; ++j) A[k][j] = sums[4 * k + j];
+                    b[k] = sums[k < 3 ? 4 * (k + 1) : 9];
+                }
+                const float3 nf = lsNormal(A, b);
+                st3(nrm, i, mk(double(nf.x), double(nf.y), double(nf.z)));
+            }
+            __syncwarp();
+        }
+        if (err) atomicOr(errOut, err);
+        return;
+    }
     for (int i = spreadFirst(); i < nm; i += spreadStride()) {
         const int c = mixed[i];
         const int32_t* st;
@@ -739,6 +804,22 @@ __device__ __forceinline__ v3f pointValueF(const DevMesh& m, int p, const double
     return r;
 }
 
+// The weights of r in the tetrahedron (0, e1, e2, e3), w0 of its apex, and the
+// least of them; false for a flat tetrahedron.
+__device__ __forceinline__ bool tetWeightsF(v3f r, v3f e1, v3f e2, v3f e3, float& w0, float& w1, float& w2, float& w3,
+                                            float& mn) {
+    const v3f c23 = crossf(e2, e3);
+    const float det = dotf(e1, c23);
+    if (!(fabsf(det) > 0.f)) return false;
+    const float id = 1.f / det;
+    w1 = dotf(r, c23) * id;
+    w2 = dotf(e1, crossf(r, e3)) * id;
+    w3 = dotf(e1, crossf(e2, r)) * id;
+    w0 = ((1.f - w1) - w2) - w3;
+    mn = fminf(fminf(w0, w1), fminf(w2, w3));
+    return true;
+}
+
 __device__ v3f interpolateUF(const DevMesh& m, int c, d3 x, const double* U, const double* Ub) {
     const d3 a = ld3(m.C, c);
     const v3f r = toF(x - a);
@@ -753,15 +834,8 @@ __device__ v3f interpolateUF(const DevMesh& m, int c, d3 x, const double* U, con
         for (int i = 1; i + 1 < n; ++i) {
             const int gi = m.fPts[q0 + i], gj = m.fPts[q0 + i + 1];
             const v3f e2 = toF(ld3(m.pts, gi) - a), e3 = toF(ld3(m.pts, gj) - a);
-            const v3f c23 = crossf(e2, e3);
-            const float det = dotf(e1, c23);
-            if (!(fabsf(det) > 0.f)) continue;
-            const float id = 1.f / det;
-            const float w1 = dotf(r, c23) * id;
-            const float w2 = dotf(e1, crossf(r, e3)) * id;
-            const float w3 = dotf(e1, crossf(e2, r)) * id;
-            const float w0 = ((1.f - w1) - w2) - w3;
-            const float mn = fminf(fminf(w0, w1), fminf(w2, w3));
+            float w0, w1, w2, w3, mn;
+            if (!tetWeightsF(r, e1, e2, e3, w0, w1, w2, w3, mn)) continue;
             // inside up to FP32 rounding of the weights
             const bool inside = mn >= -1e-6f;
             if (mn > bestMin || inside) {
@@ -789,15 +863,165 @@ __device__ v3f interpolateUF(const DevMesh& m, int c, d3 x, const double* U, con
 }
 
 // Un0 of every cut cell and the list of its downwind faces (advection.C:
-// 131-174), as the plain form's kernel, with the interpolation above.
-__global__ void __launch_bounds__(128) kInterfaceUn0Mixed(DevMesh m, const int* __restrict__ mixed,
-                                                          const int* __restrict__ nMixed,
-                                                          const int8_t* __restrict__ mStatus,
-                                                          const double* __restrict__ nrm,
-                                                          const double* __restrict__ icArr,
-                                                          const double* __restrict__ U, const double* __restrict__ Ub,
-                                                          const double* __restrict__ phi, double* __restrict__ un0,
-                                                          int2* __restrict__ dwList, int* __restrict__ dwCount) {
+// 131-174), as the plain form's kernel, with the interpolation above.  On
+// shorter lists eight lanes take a cell, four cells a warp: on its faces'
+// tetrahedra (the first that holds x, else the one with the largest least
+// weight), on the cells of that one's points, on the nine sums over them (the
+// same fused operations in the same order).  Kernel time, a thread per cell
+// against eight lanes: hexahedra 365 cells 29 / 12 us, 12,394 43 / 20, 30,189 43 /
+// 32, 39,937 47 / 43, 60,750 53 / 58; cells of two sizes (1,755) 73 / 20;
+// tetrahedra 6,299 36 / 16.
+constexpr int kUn0MixedGroup = 300;  // cells per SM
+constexpr int kUn0MixedThreads = 128;
+__global__ void __launch_bounds__(kUn0MixedThreads) kInterfaceUn0Mixed(
+    DevMesh m, const int* __restrict__ mixed, const int* __restrict__ nMixed, const int8_t* __restrict__ mStatus,
+    const double* __restrict__ nrm, const double* __restrict__ icArr, const double* __restrict__ U,
+    const double* __restrict__ Ub, const double* __restrict__ phi, double* __restrict__ un0,
+    int2* __restrict__ dwList, int* __restrict__ dwCount, int groupMax) {
+    if (*nMixed <= groupMax) {
+        constexpr unsigned kAll = 0xffffffffu;
+        __shared__ float rowS[kUn0MixedThreads / 8][12][9];  // weights of three points' cells, velocity components
+        const int nm = *nMixed, lane = threadIdx.x & 31, l = lane & 7, g = lane >> 3, base = lane & 24;
+        float(*row)[9] = rowS[threadIdx.x >> 3];
+        const int warps = gridDim.x * (kUn0MixedThreads / 32);
+        for (int q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; 4 * q < nm; q += warps) {
+            const int i = 4 * q + g;
+            const bool act = i < nm && mStatus[i] == 0;
+            const int c = act ? mixed[i] : 0;
+            const int k0 = act ? m.cOff[c] : 0, k1 = act ? m.cOff[c + 1] : 0;
+            const d3 a = ld3(m.C, c);
+            const v3f r = toF((act ? ld3(icArr, i) : a) - a);
+            const v3f uC = toF(ld3(U, c));
+            // the lane's faces: downwind or not, its first tetrahedron that
+            // holds x or its best
+            int bp0 = -1, bp1 = -1, bp2 = -1, id = INT_MAX;
+            float bw0 = 0.f, bw1 = 0.f, bw2 = 0.f, bw3 = 0.f, bestMin = -3.0e38f;
+            bool found = false;
+            for (int kb = 0; __any_sync(kAll, k0 + kb < k1); kb += 8) {
+                const int k = k0 + kb + l;
+                const int f = k < k1 ? m.cFaces[k] : 0;
+                bool down = false;
+                if (k < k1) {
+                    const long long ph = bitsOf(phi[f]);
+                    const bool owned = f >= m.nfi || m.own[f] == c;
+                    down = owned ? nonNegBits(ph)
+                                 : (!nonNegBits(ph) && (ph & 0x7fffffffffffffffLL) <= 0x7ff0000000000000LL);
+                }
+                const unsigned who = __ballot_sync(kAll, down);
+                int at = 0;
+                if (lane == 0 && who) at = atomicAdd(dwCount, __popc(who));
+                if (k < k1 && !found) {
+                    const int q0 = m.fOff[f], n = m.fOff[f + 1] - q0;
+                    const int g0 = m.fPts[q0];
+                    const v3f e1 = toF(ld3(m.pts, g0) - a);
+                    int gj = m.fPts[q0 + 1];
+                    v3f e3 = toF(ld3(m.pts, gj) - a);
+                    for (int t = 1; t + 1 < n && !found; ++t) {
+                        const int gi = gj;
+                        const v3f e2 = e3;
+                        gj = m.fPts[q0 + t + 1];
+                        e3 = toF(ld3(m.pts, gj) - a);
+                        float w0, w1, w2, w3, mn;
+                        if (!tetWeightsF(r, e1, e2, e3, w0, w1, w2, w3, mn)) continue;
+                        found = mn >= -1e-6f;
+                        if (mn > bestMin || found) {
+                            bestMin = mn;
+                            id = 16 * (k - k0) + t;
+                            bp0 = g0;
+                            bp1 = gi;
+                            bp2 = gj;
+                            bw0 = w0;
+                            bw1 = w1;
+                            bw2 = w2;
+                            bw3 = w3;
+                        }
+                    }
+                }
+                at = __shfl_sync(kAll, at, 0);
+                if (down) dwList[at + __popc(who & ((1u << lane) - 1u))] = make_int2(i, f);
+            }
+            // the group's: the first that holds x, else the first of the largest
+            const bool anyFound = (__ballot_sync(kAll, found) >> base) & 0xffu;
+            float top = anyFound ? (found ? 1.f : 0.f) : bestMin;
+            const float mine = top;
+            for (int o = 4; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(kAll, top, o));
+            int first = mine == top ? id : INT_MAX;
+            const int own = first;
+            for (int o = 4; o; o >>= 1) first = min(first, __shfl_xor_sync(kAll, first, o));
+            const unsigned win = (__ballot_sync(kAll, own == first && first != INT_MAX) >> base) & 0xffu;
+            const int src = base + (win ? __ffs(win) - 1 : 0);
+            int p[3] = {__shfl_sync(kAll, bp0, src), __shfl_sync(kAll, bp1, src), __shfl_sync(kAll, bp2, src)};
+            const float w0 = __shfl_sync(kAll, bw0, src), w1 = __shfl_sync(kAll, bw1, src),
+                        w2 = __shfl_sync(kAll, bw2, src), w3 = __shfl_sync(kAll, bw3, src);
+            const bool tet = act && win != 0;
+            int at[3], end[3];
+            bool boundary[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int pt = tet ? p[k] : 0;
+                const int b0 = m.pbOff[pt], b1 = m.pbOff[pt + 1], c0 = m.pcOff[pt], c1 = m.pcOff[pt + 1];
+                boundary[k] = b1 > b0;
+                at[k] = boundary[k] ? b0 : c0;
+                end[k] = tet ? (boundary[k] ? b1 : c1) : at[k];
+            }
+            // sum k = 3 point + component on lane k, the ninth on lane 0 too
+            float sum = 0.f, sum8 = 0.f;
+            while (__any_sync(kAll, at[0] < end[0] || at[1] < end[1] || at[2] < end[2])) {
+                int cell[3];
+                bool in[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const int e = at[k] + l;
+                    in[k] = e < end[k];
+                    cell[k] = in[k] ? (boundary[k] ? m.pbFaces : m.pCells)[e] : 0;
+                    row[k][l] = in[k] ? float((boundary[k] ? m.pbW : m.pcW)[e]) : 0.f;
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const double* u = U;
+                    if (in[k]) {
+                        if (!boundary[k]) u = U + size_t(3) * cell[k];
+                        else u = Ub ? Ub + size_t(3) * (cell[k] - m.nfi) : U + size_t(3) * m.own[cell[k]];
+                    }
+                    row[3 + 3 * k][l] = float(u[0]);
+                    row[4 + 3 * k][l] = float(u[1]);
+                    row[5 + 3 * k][l] = float(u[2]);
+                }
+                __syncwarp();
+                const int pk = l / 3;
+                const int n01 = pk == 0 ? end[0] - at[0] : (pk == 1 ? end[1] - at[1] : end[2] - at[2]);
+                const int n8 = l == 0 ? end[2] - at[2] : 0;
+                for (int j = 0; j < 8; ++j) {
+                    if (j < n01) sum = fmaf(row[pk][j], row[3 + l][j], sum);
+                    if (j < n8) sum8 = fmaf(row[2][j], row[11][j], sum8);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 3; ++k) at[k] = min(at[k] + 8, end[k]);
+            }
+            v3f v[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                v[k].x = __shfl_sync(kAll, sum, base + ((3 * k) & 7));
+                v[k].y = __shfl_sync(kAll, sum, base + ((3 * k + 1) & 7));
+                v[k].z = k < 2 ? __shfl_sync(kAll, sum, base + 3 * k + 2) : __shfl_sync(kAll, sum8, base);
+            }
+            if (act && l == 0) {
+                v3f u = uC;
+                if (tet) {
+                    u = w0 * uC;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const float wk = k == 0 ? w1 : (k == 1 ? w2 : w3);
+                        u = fv(fmaf(wk, v[k].x, u.x), fmaf(wk, v[k].y, u.y), fmaf(wk, v[k].z, u.z));
+                    }
+                }
+                const d3 n = ld3(nrm, i);
+                un0[i] = double(u.x) * n.x + double(u.y) * n.y + double(u.z) * n.z;
+            }
+        }
+        return;
+    }
     const int nm = *nMixed;
     const int lane = threadIdx.x & 31;
     const int stride = spreadStride();
@@ -841,7 +1065,8 @@ static void planeSolveMixedAll(const DevMesh& m, const PlaneArgs& p, cudaStream_
 }
 
 void launchLsNormalMixed(const StepArgs& a, cudaStream_t st) {
-    kLsNormalMixed<<<residentGridM(kLsNormalMixed, 128), 128, 0, st>>>(a.m, a.aCur, a.mixed, a.nMixed, a.nrm, a.err);
+    kLsNormalMixed<<<residentGridM(kLsNormalMixed, 128), 128, 0, st>>>(a.m, a.aCur, a.mixed, a.nMixed, a.nrm,
+                                                                        kLsMixedGroup * smCount(), a.err);
 }
 
 void launchPlaneSolveMixed(const StepArgs& a, bool boxes, cudaStream_t st) {
@@ -861,7 +1086,8 @@ void launchPlaneSolveMixed(const StepArgs& a, bool boxes, cudaStream_t st) {
 
 void launchInterfaceUn0Mixed(const StepArgs& a, cudaStream_t st) {
     kInterfaceUn0Mixed<<<residentGridM(kInterfaceUn0Mixed, 128), 128, 0, st>>>(
-        a.m, a.mixed, a.nMixed, a.mStatus, a.nrm, a.icArr, a.U, a.Ub, a.phi, a.un0, a.dwList, a.dwCount);
+        a.m, a.mixed, a.nMixed, a.mStatus, a.nrm, a.icArr, a.U, a.Ub, a.phi, a.un0, a.dwList, a.dwCount,
+        kUn0MixedGroup * smCount());
 }
 
 void launchInterfaceFacesMixed(const StepArgs& a, cudaStream_t st) {

@@ -112,6 +112,7 @@ struct simplic_handle {
     double* un0 = nullptr;
     int2* dwList = nullptr;
     int* dwCount = nullptr;
+    int* stepCounters = nullptr;  // the counters zeroed at the start of an advect, in one block
     uint32_t* devErr = nullptr;
     BoundBuffers bb{};
     RdfBuffers rdf{};  // isoRDF orientation only
@@ -657,6 +658,10 @@ int uploadMesh(simplic_handle* h, const simplic_mesh_desc* d, const HostMesh& hm
     return SIMPLIC_OK;
 }
 
+// dwCount, ovCount, barCount, info, ctl: each from a 128-byte line of its own
+// on, so that one memset (about 1.5 us of a step's 200) does for all five.
+constexpr int kStepCounters = 128 + kCtlSize;
+
 int allocState(simplic_handle* h) {
     const int nc = h->m.nc, nf = h->m.nf;
     h->nb = (nc + 255) / 256;
@@ -676,8 +681,9 @@ int allocState(simplic_handle* h) {
     h->un0 = M.alloc<double>(nc);
     // every face is downwind of at most one cell: nf entries always suffice
     h->dwList = M.alloc<int2>(nf);
-    h->dwCount = M.alloc<int>(1);
-    if (!h->un0 || !h->dwList || !h->dwCount)
+    h->stepCounters = M.alloc<int>(kStepCounters);
+    h->dwCount = h->stepCounters;
+    if (!h->un0 || !h->dwList || !h->stepCounters)
         return fail(h, SIMPLIC_ERR_CUDA, "cudaMalloc failed (plane scratch)");
     h->dvfI = M.alloc<double>(nf);
     h->alphaPhi = M.alloc<double>(nf);
@@ -689,7 +695,7 @@ int allocState(simplic_handle* h) {
     // and an overflow is reported as a device error, never truncated
     b.ovCap = std::max(1 << 17, nc / 16);
     b.ovList = M.alloc<int>(b.ovCap);
-    b.ovCount = M.alloc<int>(2);  // [0] overshooting cells, [1] listed (bounding-set) cells
+    b.ovCount = h->stepCounters + 32;  // [0] overshooting cells, [1] listed (bounding-set) cells
     b.candCap = 2 * b.ovCap;
     b.cand = M.alloc<int>(b.candCap);
     b.candIdx = M.alloc<int>(nc);
@@ -704,8 +710,8 @@ int allocState(simplic_handle* h) {
     b.modStamp = M.alloc<int>(nf);
     b.modCap = std::max(1 << 20, 4 * b.candCap);
     b.modList = M.alloc<int>(b.modCap);
-    b.ctl = M.alloc<int>(kCtlSize);
-    b.barCount = M.alloc<unsigned>(1);
+    b.ctl = h->stepCounters + 128;
+    b.barCount = reinterpret_cast<unsigned*>(h->stepCounters + 64);
     b.barGen = M.alloc<unsigned>(1);
     b.spinLimit = kBarrierSpins;
     b.barrierExtra = 0;
@@ -718,7 +724,7 @@ int allocState(simplic_handle* h) {
             b.spinLimit = spins;
         }
     }
-    b.info = M.alloc<int>(8);
+    b.info = h->stepCounters + 96;
     b.actList = M.alloc<int>(b.candCap);
     b.recBytes = int(boundRecordBytes(h->m.maxCellFaces));
     b.rec = M.alloc<uint8_t>(size_t(b.candCap) * b.recBytes);
@@ -745,9 +751,8 @@ int allocState(simplic_handle* h) {
     CK(h, cudaMemsetAsync(b.cellClaim, 0, sizeof(int) * nc, h->stream));
     CK(h, cudaMemsetAsync(b.faceStamp, 0, sizeof(int) * nf, h->stream));
     CK(h, cudaMemsetAsync(b.readyQ, 0, sizeof(unsigned long long) * b.candCap, h->stream));
-    CK(h, cudaMemsetAsync(b.barCount, 0, sizeof(unsigned), h->stream));
+    CK(h, cudaMemsetAsync(h->stepCounters, 0, sizeof(int) * kStepCounters, h->stream));
     CK(h, cudaMemsetAsync(b.barGen, 0, sizeof(unsigned), h->stream));
-    CK(h, cudaMemsetAsync(b.info, 0, sizeof(int) * 8, h->stream));
     if (h->ctrl.orientation_method == SIMPLIC_ORIENTATION_ISO_RDF) {
         RdfBuffers& r = h->rdf;
         r.rdf = M.alloc<double>(nc);
@@ -913,12 +918,8 @@ int runAdvect(simplic_handle* h, const simplic_step_inputs* in, const double* aO
     nextEvents(h, 1);
     CK(h, cudaEventRecord(h->events[evIdx].a, h->stream));
     if (a.cutMask) CK(h, cudaMemsetAsync(a.cutMask, 0, h->m.nf, h->stream));
-    CK(h, cudaMemsetAsync(h->bb.ovCount, 0, 2 * sizeof(int), h->stream));
-    CK(h, cudaMemsetAsync(h->dwCount, 0, sizeof(int), h->stream));
-    CK(h, cudaMemsetAsync(h->bb.ctl, 0, sizeof(int) * kCtlSize, h->stream));
-    CK(h, cudaMemsetAsync(h->bb.info, 0, sizeof(int) * 8, h->stream));
-    // a barrier that timed out leaves its arrival count behind
-    CK(h, cudaMemsetAsync(h->bb.barCount, 0, sizeof(unsigned), h->stream));
+    // (among them the grid barrier's count, which a barrier that timed out leaves behind)
+    CK(h, cudaMemsetAsync(h->stepCounters, 0, sizeof(int) * kStepCounters, h->stream));
     if (h->ctrl.precision != SIMPLIC_PRECISION_PLAIN_FP64) {
         timedLaunch(h, kKFluxUn0, [&] { launchInterfaceUn0Mixed(a, h->stream); });
         timedLaunch(h, kKFluxFaces, [&] { launchInterfaceFacesMixed(a, h->stream); });

@@ -17,9 +17,10 @@ namespace simplic {
 
 // v / s for the three components: one division for 1/s, then the
 // correctly rounded quotients through it (divByRecip), the same results.
+template <bool INTS = true>
 __device__ __forceinline__ d3 divBy(d3 v, double s) {
     const double y = 1.0 / s;
-    return mk(divByRecip(v.x, s, y), divByRecip(v.y, s, y), divByRecip(v.z, s, y));
+    return mk(divByRecip<INTS>(v.x, s, y), divByRecip<INTS>(v.y, s, y), divByRecip<INTS>(v.z, s, y));
 }
 
 // OpenFOAM face::centre (triangle direct; otherwise area-weighted fan about

@@ -111,6 +111,11 @@ __device__ __forceinline__ bool dotNonNegative(d3 a, d3 b) {
     return dot(a, b) >= 0.0;
 }
 
+// Quotients on the integer pipe for hexahedra, whose warps fill the FP64 pipe;
+// the larger classes have few cells and long chains (divByRecip).
+template <class K>
+constexpr bool kIntDiv = K::kFaces == 6;
+
 // x / n for a small count n: exact scaling for powers of two, else the
 // correctly rounded quotient through 1 / n (5 operations instead of a
 // division's 9).
@@ -118,13 +123,15 @@ __constant__ double kInvCount[33] = {
     0.0,      1.0 / 1,  1.0 / 2,  1.0 / 3,  1.0 / 4,  1.0 / 5,  1.0 / 6,  1.0 / 7,  1.0 / 8,  1.0 / 9,  1.0 / 10,
     1.0 / 11, 1.0 / 12, 1.0 / 13, 1.0 / 14, 1.0 / 15, 1.0 / 16, 1.0 / 17, 1.0 / 18, 1.0 / 19, 1.0 / 20, 1.0 / 21,
     1.0 / 22, 1.0 / 23, 1.0 / 24, 1.0 / 25, 1.0 / 26, 1.0 / 27, 1.0 / 28, 1.0 / 29, 1.0 / 30, 1.0 / 31, 1.0 / 32};
+template <bool INTS>
 __device__ __forceinline__ double divCount1(double x, int n) {
     if (n > 32) return x / double(n);
     const double y = kInvCount[n];
-    return (n & (n - 1)) == 0 ? x * y : divByRecip(x, double(n), y);
+    return (n & (n - 1)) == 0 ? x * y : divByRecip<INTS>(x, double(n), y);
 }
+template <bool INTS>
 __device__ __forceinline__ d3 divCount3(d3 v, int n) {
-    return mk(divCount1(v.x, n), divCount1(v.y, n), divCount1(v.z, n));
+    return mk(divCount1<INTS>(v.x, n), divCount1<INTS>(v.y, n), divCount1<INTS>(v.z, n));
 }
 
 // fmax(fabs(x), VSMALL) on the bits
@@ -361,7 +368,7 @@ __device__ __forceinline__ void groupFan(const GroupShared<K, G>& s, int lane, i
     }
     d3 fc = p0;
     for (int i = 1; i < n; ++i) fc = fc + at(i);
-    fc = divCount3(fc, n);
+    fc = divCount3<kIntDiv<K>>(fc, n);
     d3 sumN = mk(0, 0, 0), sumAc = mk(0, 0, 0);
     double sumA = 0.0;
     d3 p = p0;
@@ -379,7 +386,7 @@ __device__ __forceinline__ void groupFan(const GroupShared<K, G>& s, int lane, i
         cen = fc;
         area = mk(0, 0, 0);
     } else {
-        cen = divBy((1.0 / 3.0) * sumAc, sumA);
+        cen = divBy<kIntDiv<K>>((1.0 / 3.0) * sumAc, sumA);
         area = mk(halfOf(sumN.x), halfOf(sumN.y), halfOf(sumN.z));
     }
 }
@@ -408,8 +415,8 @@ __device__ __forceinline__ bool groupFanFlat(const GroupShared<K, G>& s, const G
         fu = fu + pu(i);
         fv = fv + pv(i);
     }
-    fu = divCount1(fu, n);
-    fv = divCount1(fv, n);
+    fu = divCount1<kIntDiv<K>>(fu, n);
+    fv = divCount1<kIntDiv<K>>(fv, n);
     double sumN = 0.0;
     d3 sumAc = mk(0, 0, 0);
     bool neg = false, pos = false, range = true;
@@ -431,7 +438,7 @@ __device__ __forceinline__ bool groupFanFlat(const GroupShared<K, G>& s, const G
     // of one sign, the magnitudes add up to the sum's magnitude, rounding by rounding
     const double sumA = fabs(sumN);
     if (!range || (neg && pos) || bitsOf(sumA) < bitsOf(kROOTVSMALL)) return false;
-    cen = divBy((1.0 / 3.0) * sumAc, sumA);
+    cen = divBy<kIntDiv<K>>((1.0 / 3.0) * sumAc, sumA);
     area = halfOf(sumN);
     return true;
 }
@@ -591,7 +598,7 @@ __device__ __forceinline__ void groupSubCell(GroupCell<K, G>& w, bool act, bool 
         }
     }
     if (nEdge > K::kEdge) err |= kErrEdgeOverflow;
-    if (nEdge > 0) fcq = divCount1(fcq, nEdge);
+    if (nEdge > 0) fcq = divCount1<kIntDiv<K>>(fcq, nEdge);
     const d3 fc = mk(__shfl_sync(kAllLanes, fcq, w.base), __shfl_sync(kAllLanes, fcq, w.base + 1),
                      __shfl_sync(kAllLanes, fcq, w.base + 2));
     // the lane's segments
@@ -740,7 +747,7 @@ __device__ __forceinline__ void groupSubCell(GroupCell<K, G>& w, bool act, bool 
     double ceq = 0.0;
     for (unsigned mm = inF; mm; mm &= mm - 1u) ceq = ceq + s.cen[q3][w.base + __ffs(mm) - 1];
     ceq = ceq + (q3 == 0 ? ic.x : (q3 == 1 ? ic.y : ic.z));
-    ceq = divCount1(ceq, __popc(inF) + 1);
+    ceq = divCount1<kIntDiv<K>>(ceq, __popc(inF) + 1);
     const d3 cEst = mk(__shfl_sync(kAllLanes, ceq, w.base), __shfl_sync(kAllLanes, ceq, w.base + 1),
                        __shfl_sync(kAllLanes, ceq, w.base + 2));
     double pyr = 0.0;
@@ -758,9 +765,9 @@ __device__ __forceinline__ void groupSubCell(GroupCell<K, G>& w, bool act, bool 
     for (unsigned mm = inF; mm; mm &= mm - 1u) v += s.term[w.base + __ffs(mm) - 1];
     if (vol) {
         v += absAtLeastVSmall(dot(is, ic - cEst));
-        v = divByRecip(v, 3.0, 1.0 / 3.0);
+        v = divByRecip<kIntDiv<K>>(v, 3.0, 1.0 / 3.0);
         out.status = 0;
-        out.vof = divByRecip(v, w.V, w.rV);  // volume / V
+        out.vof = divByRecip<kIntDiv<K>>(v, w.V, w.rV);  // volume / V
     }
     __syncwarp();
 }
@@ -935,7 +942,7 @@ __device__ __forceinline__ int groupSignedDistance(GroupCell<K, G>& w, bool act,
             // levels that coincide take the cut at their middle, the others the cubic
             cubic = !done && !absBelow(br.lowD - br.upD, kTSMALL);
             if (!done && !cubic) distance = 0.5 * (br.lowD + br.upD);
-            deltaDistance = divByRecip(br.upD - br.lowD, 3.0, 1.0 / 3.0);
+            deltaDistance = divByRecip<kIntDiv<K>>(br.upD - br.lowD, 3.0, 1.0 / 3.0);
             phase = kEnds;
         }
         // (every group takes its first unknown end in kEnds, a second one in kEnds2)
@@ -1096,7 +1103,7 @@ __device__ __forceinline__ int teamSignedDistance(GroupCell<K, G>& w, bool act, 
             } else {
                 br.lowD = sv[lowLabel];
                 br.upD = sv[upLabel];
-                deltaDistance = divByRecip(br.upD - br.lowD, 3.0, 1.0 / 3.0);
+                deltaDistance = divByRecip<kIntDiv<K>>(br.upD - br.lowD, 3.0, 1.0 / 3.0);
                 if (absBelow(br.lowD - br.upD, kTSMALL)) {  // levels that coincide: their middle
                     distance = 0.5 * (br.lowD + br.upD);
                     phase = kFinal;

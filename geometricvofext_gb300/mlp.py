@@ -144,6 +144,7 @@ class Trainer:
         self.scratch = torch.empty((N_LAYERS + 1, WIDTH, B), dtype=bf, device=self.dev)
         self.gW = torch.zeros_like(self.W)
         self.gb = torch.zeros_like(self.b)
+        self.rows = 0  # of the last forward pass: what Z and HT hold
         self._refresh()
 
     def _refresh(self):
@@ -168,11 +169,16 @@ class Trainer:
             self.HT.data_ptr(), self.Y.data_ptr(), self.err.data_ptr(), st)
         if r != 0:
             raise RuntimeError(f"simplic_mlp_train_forward failed ({r})")
+        self.rows = X.shape[0]
         return self.Y
 
     def backward(self, X, dY, split_k=8):
-        """Gradients of all weights and biases for dL/dY (FP32 [B, 128])."""
+        """Gradients of all weights and biases for dL/dY (FP32, a row per row
+        of X), X the last forward pass's rows or the first of them."""
         X, dY = self._rows(X, self.t.bfloat16), self._rows(dY, self.t.float32)
+        # the kernels take one row count for X, dY and the forward pass's Z and HT
+        if dY.shape[0] != X.shape[0] or X.shape[0] > self.rows:
+            raise RuntimeError(f"{X.shape[0]} rows of X, {dY.shape[0]} rows of dY, {self.rows} rows of the last forward")
         st = self.t.cuda.current_stream(self.dev).cuda_stream
         r = capi.load().simplic_mlp_train_backward(
             X.data_ptr(), dY.data_ptr(), X.shape[0], self.B, self.WbT.data_ptr(), self.Z.data_ptr(),

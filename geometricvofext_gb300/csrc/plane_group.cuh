@@ -849,6 +849,7 @@ __device__ __forceinline__ bool groupLevels(GroupCell<K, G>& w, bool act, unsign
     const double* sv = s.sv[w.g];
     bool up = false, dn = false;
     float Lx = 0.f, Ly = 0.f, Lz = 0.f, far = 0.f;
+    const float V = act ? leadingFloat(w.V) : 0.f;
     if (K::kFaces == 6) {
         if (act && box && l < 6) {
             const double *pl = s.P[w.g][(box >> 3) & 7], *ph = s.P[w.g][box & 7];
@@ -858,8 +859,8 @@ __device__ __forceinline__ bool groupLevels(GroupCell<K, G>& w, bool act, unsign
             for (int k = 0; k < 3; ++k) far = fmaxf(far, fabsf(leadingFloat(pl[k])) + fabsf(leadingFloat(ph[k])));
         }
     } else if (__any_sync(kAllLanes, act && box)) {
-        // A cell that fills its bounding box up to 1e-6 of its volume (refined
-        // boxes, faces and edges split) cuts like the box, inside the margins:
+        // A cell that fills its bounding box (refined boxes, faces and edges
+        // split) cuts like the box, inside the margins:
         // kernel on a 24^3 checkerboard 0.24 -> 0.165 ms, 56^3 0.73 -> 0.49.
         static_assert(K::kFaces == 6 || K::kPts <= G, "a lane per point");
         float lo[3], hi[3];
@@ -875,15 +876,17 @@ __device__ __forceinline__ bool groupLevels(GroupCell<K, G>& w, bool act, unsign
             }
             far = fmaxf(far, __shfl_xor_sync(kAllLanes, far, o));
         }
-        const float V = act ? leadingFloat(w.V) : 0.f;
-        const float B = (hi[0] - lo[0]) * (hi[1] - lo[1]) * (hi[2] - lo[2]);
-        if (act && box && fabsf(B - V) <= 1e-6f * V) {
+        if (act && box) {
             Lx = hi[0] - lo[0];
             Ly = hi[1] - lo[1];
             Lz = hi[2] - lo[2];
         }
     }
-    if (act && l < np - 2 && fminf(Lx, fminf(Ly, Lz)) > 1e-8f * far)
+    // (alpha is compared with cut volume / V, V as the mesh gives it: the
+    // fraction of the box stands for that only where V is the box's volume, here
+    // up to 1e-6 of it)
+    const bool boxVolume = fabsf(Lx * Ly * Lz - V) <= 1e-6f * V;
+    if (act && boxVolume && l < np - 2 && fminf(Lx, fminf(Ly, Lz)) > 1e-8f * far)
         levelEstimate(nI, Lx, Ly, Lz, leadingFloat(sv[0] - sv[np - 1]), leadingFloat(sv[0] - sv[l + 1]),
                       leadingFloat(alphaI), leadingFloat(1.0 - alphaI), up, dn);
     above = w.groupBits(__ballot_sync(kAllLanes, up)) << 1;

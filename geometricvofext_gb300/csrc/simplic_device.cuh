@@ -123,16 +123,29 @@ __host__ __device__ __forceinline__ uint64_t quotOnInts(uint64_t ba, uint64_t bb
     return ((uint64_t(uint32_t(e)) << 52) + m) | ((ba ^ bb) & 0x8000000000000000ull);
 }
 
+// The same on the FP64 pipe, five instructions: the product a y corrected
+// twice by Newton steps with fused residuals (Markstein, IBM J. Res. Develop.
+// 34 (1990) 111-119: once q is within one ulp of a/b and y is the correctly
+// rounded reciprocal, r = a - b q is exact in an FMA and RN(q + r y) is the
+// correctly rounded quotient; in divByRecip's range its last bit is at least
+// 2^(ea - 1023 - 105) >= 2^-1064).
+__host__ __device__ __forceinline__ double quotNewton(double a, double b, double y) {
+#ifdef __CUDA_ARCH__
+    const double q0 = __dmul_rn(a, y);
+    const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+#else
+    const double q0 = a * y;
+    const double q1 = std::fma(std::fma(-b, q0, a), y, q0);
+    return std::fma(std::fma(-b, q1, a), y, q1);
+#endif
+}
+
 // a / b rounded to nearest, given y = RN(1/b): on the integer pipe while the
 // operands, y and the quotient are normal (biased exponent fields of a and b
 // in [64, 1980], the quotient's too); other inputs (subnormals, infinities,
 // NaN, extreme ratios) take the division itself.  A zero a over a finite
-// nonzero b is the signed zero itself.  INTS false: on the FP64 pipe, five
-// instructions: the product a y corrected twice by Newton steps with fused
-// residuals (Markstein, IBM J. Res. Develop. 34 (1990) 111-119: once q is
-// within one ulp of a/b and y is the correctly rounded reciprocal, r = a - b q
-// is exact in an FMA and RN(q + r y) is the correctly rounded quotient; in the
-// range its last bit is at least 2^(ea - 1023 - 105) >= 2^-1064).  The integer
+// nonzero b is the signed zero itself.  INTS false: quotNewton.  The integer
 // form is better where the FP64 pipe is the narrow one (plane solve of
 // 128^3 hexahedra 0.665 -> 0.634 ms, its Simpson faces 0.127 -> 0.114), the
 // other where a lone warp waits for its chain (three plane solves of refined
@@ -158,12 +171,8 @@ __host__ __device__ __forceinline__ double divByRecip(double a, double b, double
         return r;
     }
     if (ea < 64 || ea > 1980 || eb < 64 || eb > 1980 || ea - eb < 64 - 1023 || ea - eb > 1980 - 1023) return a / b;
+    if (!INTS) return quotNewton(a, b, y);
 #ifdef __CUDA_ARCH__
-    if (!INTS) {
-        const double q0 = __dmul_rn(a, y);
-        const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-        return __fma_rn(__fma_rn(-b, q1, a), y, q1);
-    }
     return __longlong_as_double((long long)quotOnInts(uint64_t(ba), uint64_t(bb), uint64_t(__double_as_longlong(y))));
 #else
     uint64_t by;

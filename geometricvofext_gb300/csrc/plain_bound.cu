@@ -719,7 +719,8 @@ __global__ void __launch_bounds__(256, 2) kBound(StepArgs a, BoundBuffers s) {
                         : "+r"(left)
                         : "l"(s.candPending + (succ >= 0 ? succ : 0)), "r"(succ)
                         : "memory");
-                    const unsigned sm = __ballot_sync(kAll, succ >= 0);  // (everybody has read the record)
+                    const unsigned sm = __ballot_sync(kAll, succ >= 0);
+                    __syncwarp();  // every lane has read the record: its buffer may be filled again
                     {
                         int b = 0;
                         for (unsigned mm = sm; mm && b < nBuf; mm &= mm - 1u, ++b)

@@ -569,8 +569,9 @@ __device__ __forceinline__ void groupSubCell(GroupCell<K, G>& w, bool act, bool 
     out.status = fullyEmpty ? 1 : -1;
     out.vof = fullyEmpty ? 0.0 : 1.0;
     const bool cut = act && !fullySub && !fullyEmpty;
-    if (!__any_sync(kAllLanes, cut)) return;
-    __syncwarp();
+    const bool anyCut = __any_sync(kAllLanes, cut);
+    __syncwarp();  // (also before the next call writes dist)
+    if (!anyCut) return;
     // calcInterfaceCentreAndArea (cutCell.C:37-100).  A face the plane cuts
     // has two edge points, one segment (plain: all of the warp's do); warped
     // or concave faces may have more.

@@ -637,6 +637,11 @@ __device__ __forceinline__ double faceDVf(const DevMesh& m, const UpdateArgs& u,
 //     cell across from shared memory; the fluxes through the tile's low sides
 //     are one more flux for two thirds of the threads (3.6 fluxes per cell
 //     instead of 6).
+// An empty cell's three fluxes, for the cells across, are zeros, or NaN where
+// phi is not finite.  HANDED: alpha was handed over again after the interface
+// was found, so an empty cell or its neighbour may have been cut then: the
+// fluxes downwind of a cut cell are its Simpson values all the same (apart
+// because the reads of status take the spread case below from 1.00 to 1.06 ms).
 // Other meshes take one thread per cell in cell order (TX = TY = TZ = 0).
 // One GB300, before -> with the products on integers -> with tiles: 128^3 in
 // the middle of the deformation run 0.222 -> 0.174 -> 0.156 ms, 256^3 with
@@ -650,7 +655,7 @@ template <int TX, int TY, int TZ>
 struct UpdateBlock {
     static constexpr int kThreads = TX ? TX * TY * TZ : 256;
 };
-template <int TX, int TY, int TZ>
+template <int TX, int TY, int TZ, bool HANDED>
 __global__ void __launch_bounds__((UpdateBlock<TX, TY, TZ>::kThreads), (1280 / UpdateBlock<TX, TY, TZ>::kThreads))
     kUpdate(DevMesh m, UpdateArgs u) {
     constexpr bool kTile = TX > 0;
@@ -680,6 +685,7 @@ __global__ void __launch_bounds__((UpdateBlock<TX, TY, TZ>::kThreads), (1280 / U
     bool work = false, interior = false;
     int k0 = 0, k1 = 0;  // slots in memory; an interior lattice cell: k0 its latticeBase
     double ao = 0.0, ac = 0.0;
+    const auto highSide = [&](int nb) { return nb == c + 1 ? 0 : (nb == c + m.latNx ? 1 : 2); };  // an owned face's axis
     if (valid) {
         // The face-slot records: from the lattice formula for the interior
         // cells of a lattice mesh (no addressing read), else the first
@@ -761,7 +767,7 @@ __global__ void __launch_bounds__((UpdateBlock<TX, TY, TZ>::kThreads), (1280 / U
     if (kTile) {
         sWork[tid] = interior && work;
         if (!__syncthreads_or(work)) return;
-        // each interior cell's +x, +y, +z fluxes (zero next to an empty cell)
+        // each interior cell's +x, +y, +z fluxes, and an empty cell's
         if (interior && work) {
 #pragma unroll 1
             for (int d = 0; d < 3; ++d) {
@@ -771,8 +777,28 @@ __global__ void __launch_bounds__((UpdateBlock<TX, TY, TZ>::kThreads), (1280 / U
                 u.alphaPhi[f] = q;
             }
         } else if (!work) {
+            const auto empty = [&](int f) {  // phi 0
+                const bool finite = (bitsOf(u.phi[f]) & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
+                return __longlong_as_double(finite ? 0LL : 0x7fffffffffffffffLL);
+            };
+            if (interior) {
 #pragma unroll
-            for (int d = 0; d < 3; ++d) sDv[d][tid] = 0.0;
+                for (int d = 0; d < 3; ++d) sDv[d][tid] = empty(k0 + d);
+            }
+#pragma unroll 1
+            for (int q = k0; q < k1; ++q) {  // (a boundary cell)
+                const int2 s = m.cSlot[q];
+                if (s.x >= 0 && s.y >= 0) sDv[highSide(s.x)][tid] = empty(s.y);
+            }
+            if (HANDED && valid) {
+                stC = u.status[c];
+#pragma unroll 1
+                for (int q = 6 * c; q < 6 * c + 6; ++q) {
+                    const int2 s = m.cSlot[q];
+                    if (s.x < 0 || s.y < 0) continue;
+                    if ((nonNegBits(bitsOf(u.phi[s.y])) ? stC : u.status[s.x]) == 0) sDv[highSide(s.x)][tid] = u.dvfI[s.y];
+                }
+            }
         }
         // the fluxes through the tile's low sides, a thread each
         if (tid < kHz + kHy + kHx) {
@@ -809,7 +835,7 @@ __global__ void __launch_bounds__((UpdateBlock<TX, TY, TZ>::kThreads), (1280 / U
             if (own) {
                 u.alphaPhi[f] = ap;
                 sum += dv;
-                if (kTile && s.x >= 0) sDv[s.x == c + 1 ? 0 : (s.x == c + m.latNx ? 1 : 2)][tid] = dv;
+                if (kTile && s.x >= 0) sDv[highSide(s.x)][tid] = dv;
             } else {
                 sum -= dv;
             }
@@ -972,7 +998,8 @@ static void launchUpdateTiles(const StepArgs& a, const UpdateArgs& u, cudaStream
     constexpr int kThreads = TX * TY * TZ;
     static_assert(TX * TY + TX * TZ + TY * TZ <= kThreads, "at most one low side per thread");
     const dim3 grid((a.m.latNx + TX - 1) / TX, (a.m.latNy + TY - 1) / TY, (a.m.latNz + TZ - 1) / TZ);
-    kUpdate<TX, TY, TZ><<<grid, kThreads, 0, st>>>(a.m, u);
+    if (a.handed) kUpdate<TX, TY, TZ, true><<<grid, kThreads, 0, st>>>(a.m, u);
+    else kUpdate<TX, TY, TZ, false><<<grid, kThreads, 0, st>>>(a.m, u);
 }
 
 void launchUpdate(const StepArgs& a, cudaStream_t st) {
@@ -984,7 +1011,7 @@ void launchUpdate(const StepArgs& a, cudaStream_t st) {
         launchUpdateTiles<8, 4, 4>(a, u, st);
         return;
     }
-    kUpdate<0, 0, 0><<<(a.m.nc + 255) / 256, 256, 0, st>>>(a.m, u);
+    kUpdate<0, 0, 0, false><<<(a.m.nc + 255) / 256, 256, 0, st>>>(a.m, u);
 }
 
 void launchBruteForce(const StepArgs& a, cudaStream_t st) {

@@ -895,8 +895,9 @@ int runReconstruct(simplic_handle* h) {
     return SIMPLIC_OK;
 }
 
-// advect from aBuf[cur] into aBuf[1-cur]; in holds device pointers
-int runAdvect(simplic_handle* h, const simplic_step_inputs* in, const double* aOld) {
+// advect from aBuf[cur] into aBuf[1-cur]; in holds device pointers; handed:
+// aBuf[cur] was filled again after the reconstruct
+int runAdvect(simplic_handle* h, const simplic_step_inputs* in, const double* aOld, bool handed) {
     if (!h->reconstructed) return fail(h, SIMPLIC_ERR_STATE, "advect called before reconstruct");
     if (!(in->dt > 0.0) || !std::isfinite(in->dt)) return fail(h, SIMPLIC_ERR_INVALID_ARGUMENT, "dt must be > 0");
     if (!in->phi || !in->U) return fail(h, SIMPLIC_ERR_INVALID_ARGUMENT, "phi and U are required");
@@ -904,6 +905,7 @@ int runAdvect(simplic_handle* h, const simplic_step_inputs* in, const double* aO
     a.aCur = h->aBuf[h->cur];
     a.aOld = aOld ? aOld : h->aBuf[h->cur];
     a.aNew = h->aBuf[1 - h->cur];
+    a.handed = handed;
     a.phi = in->phi;
     a.U = in->U;
     a.Ub = in->U_boundary;
@@ -1085,7 +1087,7 @@ int simplic_reconstruct_resident(simplic_handle* h) {
 
 int simplic_advect_resident(simplic_handle* h, const simplic_step_inputs* in) {
     if (!h || !in) return fail(h, SIMPLIC_ERR_INVALID_ARGUMENT, "NULL argument");
-    return runAdvect(h, in, nullptr);
+    return runAdvect(h, in, nullptr, false);
 }
 
 const double* simplic_alpha_device(const simplic_handle* h) { return h ? h->aBuf[h->cur] : nullptr; }
@@ -1161,7 +1163,7 @@ int simplic_advect(simplic_handle* h, double* alpha, const double* alpha_old, co
         CK(h, cudaMemcpyAsync(h->sSu, in->Su, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
         d.Su = h->sSu;
     }
-    if ((r = runAdvect(h, &d, aOld))) return r;
+    if ((r = runAdvect(h, &d, aOld, !(in->flags & SIMPLIC_ALPHA_UNCHANGED)))) return r;
     CK(h, cudaMemcpyAsync(alpha, h->aBuf[h->cur], sizeof(double) * nc, cudaMemcpyDeviceToHost, s));
     return checkDeviceErrors(h);
 }

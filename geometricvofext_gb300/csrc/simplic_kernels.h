@@ -18,6 +18,7 @@ struct StepArgs {
     const double* aCur;   // alpha used for classification and upwind fluxes
     const double* aOld;   // alpha.oldTime()
     double* aNew;         // output of advect
+    bool handed;          // aCur was handed over again after the interface was found in it
     // per-step inputs
     const double* phi;
     const double* U;

@@ -515,7 +515,9 @@ int uploadMesh(simplic_handle* h, const simplic_mesh_desc* d, const HostMesh& hm
         if (cOff[c + 1] - cOff[c] != m.uniformFaces) m.uniformFaces = 0;
     // a single-block lattice: the dimensions from cell 0's owned neighbours
     // (+x = 1, +y = nx, +z = nx ny), accepted only if every interior cell's
-    // slot records are those latticeSlots gives
+    // slot records are those latticeSlots gives and every boundary cell owns
+    // faces to its lattice neighbours alone (the tiled update keeps a cell's
+    // fluxes by axis)
     m.latNx = m.latNy = m.latNz = 0;
     m.latDivLayer = m.latDivNx = FastDiv{0u, 0};
     if (m.uniformFaces == 6 && nc >= 27) {
@@ -526,15 +528,21 @@ int uploadMesh(simplic_handle* h, const simplic_mesh_desc* d, const HostMesh& hm
             const int nx = nb[1], ny = nb[2] / nb[1];
             const int nz = (ny > 0 && nc % (nx * ny) == 0) ? nc / (nx * ny) : 0;
             bool ok = nz >= 3 && ny >= 3 && nx >= 3;
-            // the device derives a cell's lattice position by multiplications
-            // (latticeSlotsFast); every cell is checked with that same code
+            // (the position of a cell by multiplications instead of divisions: latticeSlotsFast)
             const FastDiv dLayer = makeFastDiv(uint32_t(nx) * uint32_t(ny)), dNx = makeFastDiv(uint32_t(nx));
             for (int c = 0; ok && c < nc; ++c) {
                 int2 sl[6], sr[6];
                 const bool in = latticeSlotsFast(c, nx, ny, nz, dLayer, dNx, sl);
                 ok = in == latticeSlots(c, nx, ny, nz, sr);
-                if (!ok || !in) continue;
-                for (int q = 0; q < 6 && ok; ++q) ok = sl[q].x == cSlot[6 * size_t(c) + q].x && sl[q].y == cSlot[6 * size_t(c) + q].y;
+                for (int q = 0; q < 6 && ok; ++q) {
+                    const int2 has = cSlot[6 * size_t(c) + q];
+                    if (in) {
+                        ok = sl[q].x == has.x && sl[q].y == has.y;
+                    } else if (has.x >= 0 && has.y >= 0) {  // an owned internal face of a boundary cell
+                        ok = (has.x == c + 1 && c % nx < nx - 1) || (has.x == c + nx && c / nx % ny < ny - 1) ||
+                             has.x == c + nx * ny;
+                    }
+                }
             }
             if (ok) {
                 m.latNx = nx;

@@ -56,9 +56,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = "SimPLIC cell-steps/s: plain FP64 vs learned-normal mixed at equal shape error"
 UNIT = "cell-steps/s"
-# algorithmic bytes per cell-step of the bulk update (alpha_old, alpha_new,
-# V, and per face phi, alphaPhi, owner+neighbour: 24 + 3*24)
-BULK_BYTES_PER_CELL = 96.0
+# algorithmic bytes per cell-step of the bulk update on a lattice: alpha in and
+# out, and phi and alphaPhi of three faces (the face slots are computed, and V
+# is read only by cells that are not in an empty neighbourhood)
+BULK_BYTES_PER_CELL = 64.0
 # ncu summary of the update kernel: "dram_bytes_per_cell <value>" and the
 # workload line, read for the roofline's traffic figure
 UPDATE_PROFILE = os.path.join(ROOT, "profiles", "simplic_update_256_dram.md")
@@ -451,7 +452,7 @@ def run_ours(args):
             "bytes_per_launch": upd_bytes, "peak_source": f"{src} hbm_gbs (burst copy)",
             "timing": "CUDA events around each update launch in the kernel pass (K steps after the window)",
             "dominant_kernel": dominant,
-            # whole step against HBM: the 96 B/cell bulk bytes over the step time
+            # whole step against HBM: the bulk bytes over the step time
             "step_achieved_gbs": upd_bytes / (step_ms * 1e-3) / 1e9,
             "step_frac": upd_bytes / (step_ms * 1e-3) / 1e9 / hbm,
             "kernel_ms_per_step": {k: round(v / args.steps, 4) for k, v in ktot.items()},

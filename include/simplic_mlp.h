@@ -51,9 +51,10 @@ int simplic_mlp_forward(const void* X, const int32_t* M, int32_t maxRows, const 
  * [3][128][ld] (pre-activations and transposed activations of the hidden
  * layers), Y and dY FP32 [ld][128], scratch BF16 [5][128][ld].  X is
  * contiguous.  All bases 16-byte aligned.  The backward pass needs M a
- * multiple of 64 and ld of 8; gW FP32 [4][128][128] and gb FP32 [4][128] are
- * overwritten; splitK is the least number of parts the rows are split into
- * for the weight gradients. */
+ * multiple of 64 and ld of 8, M rows of dY as of X, and at most the rows that
+ * the forward pass filled Z and HT with; gW FP32 [4][128][128] and gb FP32
+ * [4][128] are overwritten; splitK is the least number of parts the rows are
+ * split into for the weight gradients. */
 int simplic_mlp_train_forward(const void* X, int32_t M, int32_t ld, const void* W, const float* b, float* Z, void* HT,
                               float* Y, uint32_t* err, void* stream);
 int simplic_mlp_train_backward(const void* X, const float* dY, int32_t M, int32_t ld, const void* WT, const float* Z,

@@ -643,14 +643,14 @@ __device__ __forceinline__ double faceDVf(const DevMesh& m, const UpdateArgs& u,
 // fluxes downwind of a cut cell are its Simpson values all the same (apart
 // because the reads of status take the spread case below from 1.00 to 1.06 ms).
 // Other meshes take one thread per cell in cell order (TX = TY = TZ = 0).
-// One GB300, before -> with the products on integers -> with tiles: 128^3 in
-// the middle of the deformation run 0.222 -> 0.174 -> 0.156 ms, 256^3 with
-// alpha spread over the mesh 2.05 -> 1.76 -> 1.07 ms (0.28 -> 0.29 -> 0.25 ms
-// in its first steps); 45^3 x 6 tetrahedra (no lattice) 0.048 -> 0.039 ms.
-// The FP64 pipe is 63% busy then, the issue slots 55%.  Other tiles, same
-// two cases: 8 x 8 x 4 0.168 and 1.14, 16 x 4 x 4 0.174 and 1.24, 32 x 4 x 2
-// 0.192 and 1.50 (more sides, or more warps at a barrier); 8 or 12 blocks of
-// 128 per SM instead of 10 lose 0.04 ms in the first steps.
+// One GB300, before -> now: 128^3 in the middle of the deformation run 0.222 ->
+// 0.160 ms, 256^3 with alpha spread over the mesh 2.05 -> 1.01 ms (0.28 -> 0.24
+// ms in its first steps); 45^3 x 6 tetrahedra (no lattice) 0.048 -> 0.039 ms.
+// In that 128^3 step the FP64 pipe is 55% busy, the ALU pipe 61%, the issue
+// slots 58%.  Other tiles, 128^3 and spread 256^3 (0.156 and 1.07 ms then): 8 x
+// 8 x 4 0.168 and 1.14, 16 x 4 x 4 0.174 and 1.24, 32 x 4 x 2 0.192 and 1.50
+// (more sides, or more warps at a barrier); 8 or 12 blocks of 128 per SM
+// instead of 10 lose 0.04 ms in the first steps.
 template <int TX, int TY, int TZ>
 struct UpdateBlock {
     static constexpr int kThreads = TX ? TX * TY * TZ : 256;

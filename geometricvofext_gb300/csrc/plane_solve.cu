@@ -2,18 +2,14 @@
 // cutCell.C:611-799), a group of lanes per cell (plane_group.cuh).  Built
 // with -fmad=false.
 //
-// One GB300, kernel time with one thread per cell -> a group per cell -> with
-// the work left out that plane_group.cuh lists (deformation field; interface
-// cells in brackets) -> a warp per cell on short lists:
-//   24^3 hex (331) 0.861 -> 0.167 -> 0.101 -> 0.049 ms
-//   33^3 hex (617) 0.880 -> 0.224 -> 0.138 -> 0.066 ms
-//   128^3 hex (30,189) 1.451 -> 1.345 -> 0.660 ms, 0.634 with quotients on integers
-//   256^3 hex (35,452) 1.636 -> 1.628 -> 0.764 ms, 0.720
-//   96^3 warped hex (7,146) 0.985 -> 0.406 -> 0.348 ms
-//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 2.16 -> 1.56 -> 1.24 ms,
-//   then 0.71 with the classes in one launch, 0.49 with their boxes' levels
-//   settled in single precision
-// At the large sizes the FP64 pipe is about 80% busy.
+// One GB300, kernel time with one thread per cell -> now (deformation field;
+// interface cells in brackets):
+//   24^3 hex (331) 0.861 -> 0.049 ms, 33^3 (617) 0.880 -> 0.055
+//   128^3 hex (30,189) 1.451 -> 0.634, 256^3 (35,452) 1.636 -> 0.720
+//   96^3 warped hex (7,146) 0.985 -> 0.348
+//   24^3 with 2:1 refinement (755), three solves: 20.8 -> 0.49
+// In the middle of the 128^3 run the FP64 pipe is 72% busy in active cycles,
+// 64% of the kernel's time (the rest is the tail).
 #include "plane_group.cuh"
 #include "simplic_kernels.h"
 

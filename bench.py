@@ -582,7 +582,7 @@ def run_e2e(g, mesh, alpha0, flow, dt, args, dev):
             "steps": K, "path": "simplic_reconstruct + simplic_advect (host pinned buffers reused per step)",
             "ms_per_step": 1e3 * el / K, "device_ms_per_step": 1e3 * dev_s / K,
             "copy_and_host_ms_per_step": 1e3 * (el - dev_s) / K,
-            "effective_copy_gbs": (h2d + d2h) / max(1e-12, el - dev_s) / 1e9,
+            "effective_copy_gbs": K * (h2d + d2h) / max(1e-12, el - dev_s) / 1e9,
             "link_gbs": {k: round(v, 1) for k, v in bw.items()},
             "link_bound_ms_per_step": 1e3 * (h2d / (bw["h2d"] * 1e9) + d2h / (bw["d2h"] * 1e9))}
 
